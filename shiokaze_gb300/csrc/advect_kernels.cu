@@ -17,61 +17,86 @@
 // record (4 + 8), backward reads them and the input (16) and writes the
 // result (4): 32 B. Cell scalar: the same 32 B plus the fluid level set read
 // twice (8) and, on the cell passes, the 3 velocity components' two faces
-// (counted once, 12). The arithmetic is the reference's: trilinear weights
-// and sums in FP64 on every trace (three per face, two per cell), which on
-// this GPU's FP64 pipe, not DRAM, bounds the kernels.
+// (counted once, 12). The reference's arithmetic is double precision
+// throughout, and in FP64 instructions its trilinear weights and sums kept
+// the FP64 pipe 86 % busy; the kernels take each element through the
+// float-pair form of advect_fast.cuh, with the FP64 form (advect_core.cuh)
+// for the few it leaves undecided, and are bound by FP32 instruction issue
+// instead. A 256^3 smoke step (density and velocity): 40.75 ms in FP64,
+// 3.51 ms in float pairs; a 1000 x 777 2D step 1.09 ms and 0.19 ms; the same
+// bits.
 #include <algorithm>
 #include <cfloat>
 #include <cmath>
 
 #include "advect.h"
 #include "advect_core.cuh"
+#include "advect_fast.cuh"
 
 namespace gbp {
 namespace {
 
 using gba::Dims;
+using gba::Fast;
 using gba::StepArgs;
 
 constexpr int ADV_THREADS = 256;
 
 // one thread per face, blockIdx.y = component
 template <bool MAC>
-__global__ void __launch_bounds__(ADV_THREADS) adv_face_forward(StepArgs a) {
-    gba::face_forward<MAC>(a, (int)blockIdx.y, blockIdx.x * blockDim.x + threadIdx.x);
+__global__ void __launch_bounds__(ADV_THREADS) adv_face_forward(const __grid_constant__ StepArgs a,
+                                                               const __grid_constant__ Fast k) {
+    const unsigned f = blockIdx.x * blockDim.x + threadIdx.x;
+    if (blockIdx.y == 0) gba::face_forward_any<0, MAC>(a, k, f);
+    else if (blockIdx.y == 1) gba::face_forward_any<1, MAC>(a, k, f);
+    else gba::face_forward_any<2, MAC>(a, k, f);
 }
 
-__global__ void __launch_bounds__(ADV_THREADS) adv_face_backward(StepArgs a) {
-    gba::face_backward(a, (int)blockIdx.y, blockIdx.x * blockDim.x + threadIdx.x);
+__global__ void __launch_bounds__(ADV_THREADS) adv_face_backward(const __grid_constant__ StepArgs a,
+                                                                const __grid_constant__ Fast k) {
+    const unsigned f = blockIdx.x * blockDim.x + threadIdx.x;
+    if (blockIdx.y == 0) gba::face_backward_any<0>(a, k, f);
+    else if (blockIdx.y == 1) gba::face_backward_any<1>(a, k, f);
+    else gba::face_backward_any<2>(a, k, f);
 }
 
 // one thread per cell
 template <bool MAC>
-__global__ void __launch_bounds__(ADV_THREADS) adv_cell_forward(StepArgs a) {
-    gba::cell_forward<MAC>(a, blockIdx.x * blockDim.x + threadIdx.x);
+__global__ void __launch_bounds__(ADV_THREADS) adv_cell_forward(const __grid_constant__ StepArgs a,
+                                                               const __grid_constant__ Fast k) {
+    gba::cell_forward_any<MAC>(a, k, blockIdx.x * blockDim.x + threadIdx.x);
 }
 
-__global__ void __launch_bounds__(ADV_THREADS) adv_cell_backward(StepArgs a) {
-    gba::cell_backward(a, blockIdx.x * blockDim.x + threadIdx.x);
+__global__ void __launch_bounds__(ADV_THREADS) adv_cell_backward(const __grid_constant__ StepArgs a,
+                                                                const __grid_constant__ Fast k) {
+    gba::cell_backward_any(a, k, blockIdx.x * blockDim.x + threadIdx.x);
 }
 
 // the 2D passes: one thread per face (blockIdx.y = component) or cell
 template <bool MAC>
-__global__ void __launch_bounds__(ADV_THREADS) adv2_face_forward(StepArgs a) {
-    gba::face_forward2<MAC>(a, (int)blockIdx.y, blockIdx.x * blockDim.x + threadIdx.x);
+__global__ void __launch_bounds__(ADV_THREADS) adv2_face_forward(const __grid_constant__ StepArgs a,
+                                                                const __grid_constant__ Fast k) {
+    const unsigned f = blockIdx.x * blockDim.x + threadIdx.x;
+    if (blockIdx.y == 0) gba::face_forward2_any<0, MAC>(a, k, f);
+    else gba::face_forward2_any<1, MAC>(a, k, f);
 }
 
-__global__ void __launch_bounds__(ADV_THREADS) adv2_face_backward(StepArgs a) {
-    gba::face_backward2(a, (int)blockIdx.y, blockIdx.x * blockDim.x + threadIdx.x);
+__global__ void __launch_bounds__(ADV_THREADS) adv2_face_backward(const __grid_constant__ StepArgs a,
+                                                                 const __grid_constant__ Fast k) {
+    const unsigned f = blockIdx.x * blockDim.x + threadIdx.x;
+    if (blockIdx.y == 0) gba::face_backward2_any<0>(a, k, f);
+    else gba::face_backward2_any<1>(a, k, f);
 }
 
 template <bool MAC>
-__global__ void __launch_bounds__(ADV_THREADS) adv2_cell_forward(StepArgs a) {
-    gba::cell_forward2<MAC>(a, blockIdx.x * blockDim.x + threadIdx.x);
+__global__ void __launch_bounds__(ADV_THREADS) adv2_cell_forward(const __grid_constant__ StepArgs a,
+                                                                const __grid_constant__ Fast k) {
+    gba::cell_forward2_any<MAC>(a, k, blockIdx.x * blockDim.x + threadIdx.x);
 }
 
-__global__ void __launch_bounds__(ADV_THREADS) adv2_cell_backward(StepArgs a) {
-    gba::cell_backward2(a, blockIdx.x * blockDim.x + threadIdx.x);
+__global__ void __launch_bounds__(ADV_THREADS) adv2_cell_backward(const __grid_constant__ StepArgs a,
+                                                                 const __grid_constant__ Fast k) {
+    gba::cell_backward2_any(a, k, blockIdx.x * blockDim.x + threadIdx.x);
 }
 
 // levelset_exist (include/shiokaze/array/array_utility3.h:112-122): any
@@ -158,6 +183,7 @@ cudaError_t advect_run(AdvectWork &w, const AdvectArgs &a, cudaStream_t st, long
     StepArgs s{};
     s.g = make_dims(a.nx, a.ny, a.nz, a.dx, a.trim_narrowband);
     s.dt = a.dt;
+    const Fast k = gba::make_fast(s.g, a.dt, true);
     s.u = a.u;
     s.v = a.v;
     s.w = a.w;
@@ -173,11 +199,11 @@ cudaError_t advect_run(AdvectWork &w, const AdvectArgs &a, cudaStream_t st, long
     s.qmm = w.qmm;
     if (a.q) {
         if (a.maccormack) {
-            adv_cell_forward<true><<<blocks_for(cells), ADV_THREADS, 0, st>>>(s);
-            adv_cell_backward<<<blocks_for(cells), ADV_THREADS, 0, st>>>(s);
+            adv_cell_forward<true><<<blocks_for(cells), ADV_THREADS, 0, st>>>(s, k);
+            adv_cell_backward<<<blocks_for(cells), ADV_THREADS, 0, st>>>(s, k);
             *launches += 2;
         } else {
-            adv_cell_forward<false><<<blocks_for(cells), ADV_THREADS, 0, st>>>(s);
+            adv_cell_forward<false><<<blocks_for(cells), ADV_THREADS, 0, st>>>(s, k);
             *launches += 1;
             e = cudaMemcpyAsync(a.q, w.q0, sizeof(float) * (size_t)cells, cudaMemcpyDeviceToDevice, st);
             if (e != cudaSuccess) return e;
@@ -186,11 +212,11 @@ cudaError_t advect_run(AdvectWork &w, const AdvectArgs &a, cudaStream_t st, long
     if (!a.velocity) return cudaGetLastError();
     const dim3 fgrid(blocks_for(nfmax), 3);
     if (a.maccormack) {
-        adv_face_forward<true><<<fgrid, ADV_THREADS, 0, st>>>(s);
-        adv_face_backward<<<fgrid, ADV_THREADS, 0, st>>>(s);
+        adv_face_forward<true><<<fgrid, ADV_THREADS, 0, st>>>(s, k);
+        adv_face_backward<<<fgrid, ADV_THREADS, 0, st>>>(s, k);
         *launches += 2;
     } else {
-        adv_face_forward<false><<<fgrid, ADV_THREADS, 0, st>>>(s);
+        adv_face_forward<false><<<fgrid, ADV_THREADS, 0, st>>>(s, k);
         *launches += 1;
         float *dst[3] = {a.u, a.v, a.w};
         const long long n[3] = {nf0, nf1, nf2}, o[3] = {0, s.off1, s.off2};
@@ -211,6 +237,7 @@ cudaError_t advect_run2(AdvectWork &w, const AdvectArgs &a, cudaStream_t st, lon
     StepArgs s{};
     s.g = make_dims(a.nx, a.ny, 1, a.dx, a.trim_narrowband);
     s.dt = a.dt;
+    const Fast k = gba::make_fast(s.g, a.dt, false);
     s.u = a.u;
     s.v = a.v;
     s.w = nullptr;
@@ -226,11 +253,11 @@ cudaError_t advect_run2(AdvectWork &w, const AdvectArgs &a, cudaStream_t st, lon
     s.qmm = w.qmm;
     if (a.q) {
         if (a.maccormack) {
-            adv2_cell_forward<true><<<blocks_for(cells), ADV_THREADS, 0, st>>>(s);
-            adv2_cell_backward<<<blocks_for(cells), ADV_THREADS, 0, st>>>(s);
+            adv2_cell_forward<true><<<blocks_for(cells), ADV_THREADS, 0, st>>>(s, k);
+            adv2_cell_backward<<<blocks_for(cells), ADV_THREADS, 0, st>>>(s, k);
             *launches += 2;
         } else {
-            adv2_cell_forward<false><<<blocks_for(cells), ADV_THREADS, 0, st>>>(s);
+            adv2_cell_forward<false><<<blocks_for(cells), ADV_THREADS, 0, st>>>(s, k);
             *launches += 1;
             e = cudaMemcpyAsync(a.q, w.q0, sizeof(float) * (size_t)cells, cudaMemcpyDeviceToDevice, st);
             if (e != cudaSuccess) return e;
@@ -239,11 +266,11 @@ cudaError_t advect_run2(AdvectWork &w, const AdvectArgs &a, cudaStream_t st, lon
     if (!a.velocity) return cudaGetLastError();
     const dim3 fgrid(blocks_for(nfmax), 2);
     if (a.maccormack) {
-        adv2_face_forward<true><<<fgrid, ADV_THREADS, 0, st>>>(s);
-        adv2_face_backward<<<fgrid, ADV_THREADS, 0, st>>>(s);
+        adv2_face_forward<true><<<fgrid, ADV_THREADS, 0, st>>>(s, k);
+        adv2_face_backward<<<fgrid, ADV_THREADS, 0, st>>>(s, k);
         *launches += 2;
     } else {
-        adv2_face_forward<false><<<fgrid, ADV_THREADS, 0, st>>>(s);
+        adv2_face_forward<false><<<fgrid, ADV_THREADS, 0, st>>>(s, k);
         *launches += 1;
         e = cudaMemcpyAsync(a.u, w.v0, sizeof(float) * (size_t)nf0, cudaMemcpyDeviceToDevice, st);
         if (e == cudaSuccess)
