@@ -95,7 +95,8 @@ typedef struct gbp_params {
     int mg_smooth;          /* red-black sweeps before and after each coarse correction (default 1) */
     int mg_coarsest;        /* coarsen while any edge exceeds this (default 7) */
     double inner_tolerance; /* MIXED: relative residual of each inner solve (default 1e-3) */
-    int iterations_per_sync;/* CG iterations between host checks of convergence (default 16) */
+    int iterations_per_sync;/* CG iterations between host checks of convergence (default 16); a solve that fits the
+                               SMs' shared memory runs in one launch and checks every iteration on the device */
     double surface_tension; /* the surface_tension argument of macproject3_interface::project
                                (macpressuresolver3.cpp:85-115); 0 (default) leaves the velocity as is */
     int tma_staging;        /* MGPCG MIXED: nonzero runs the fine level's four stencil passes with their

@@ -11,6 +11,8 @@
 // update 48 and direction 24 per row.
 #include "csr_solver.h"
 
+#include "cg_persistent.cuh"
+
 namespace gbp {
 namespace {
 
@@ -225,6 +227,29 @@ cudaError_t csr_cg_run(CsrWork &w, long long n, double residual, int max_iter, i
     csr_init_kernel<<<nb, BLOCK_THREADS, 0, stream>>>(n, w.b, w.x, w.r, w.s, w.sc, w.pt, residual, max_iter);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     *launches += 1;
+    const long long per = (n + (long long)nb * BLOCK_THREADS - 1) / ((long long)nb * BLOCK_THREADS);
+    CgPersistentPlan plan;
+    if (per <= 64) plan = cg_persistent_plan(nb, (int)per, grid_blocks / 6);
+    if (plan.use) {
+        plan.args.x = w.x;
+        plan.args.r = w.r;
+        plan.args.s = w.s;
+        plan.args.sc = w.sc;
+        plan.args.pt = w.pt;
+        for (int left = max_iter; e == cudaSuccess; left -= CG_PERSISTENT_STEPS) {
+            if ((e = cg_persistent_launch(plan, cgp::CsrRows{n, w.rowstart, w.cols, w.vals}, stream)) != cudaSuccess)
+                break;
+            *launches += 1;
+            if ((e = cudaMemcpyAsync(w.host_sc, w.sc, sizeof(Scalars), cudaMemcpyDeviceToHost, stream)) != cudaSuccess ||
+                (e = cudaStreamSynchronize(stream)) != cudaSuccess)
+                return e;
+            if (w.host_sc->status == 4) return cudaErrorLaunchTimeout;
+            if (w.host_sc->done || left <= 0) return cudaSuccess;
+        }
+        // blocks that cannot be resident together (a partitioned GPU): the launched form
+        if (e != cudaErrorCooperativeLaunchTooLarge) return e;
+        cudaGetLastError();
+    }
     if (!w.graph || w.graph_n != n || w.graph_blocks != nb) {
         if (w.graph) cudaGraphExecDestroy(w.graph);
         w.graph = nullptr;
