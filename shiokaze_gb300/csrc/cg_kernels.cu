@@ -60,17 +60,18 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 6) cg_init_kernel(Grid g, Opera
                                                                 double *s, Scalars *sc, Partials *pt,
                                                                 double residual, int max_iter) {
     __shared__ double sh[BLOCK_THREADS / 32];
-    double mx = 0.0, r2 = 0.0;
+    unsigned long long mx = 0;
+    double r2 = 0.0;
     for_each_cell(g, [&](int i, int j, int k, long long c) {
         double rv = __ldg(b + c);
         if (prev) rv -= apply_A(g, A, prev, i, j, k, c);  // macpressuresolver3.cpp:228-229
         x[c] = 0.0;
         r[c] = rv;
         s[c] = rv;
-        mx = fmax(mx, fabs(rv));
+        mx = max(mx, abs_bits(rv));
         r2 = fma(rv, rv, r2);
     });
-    double bm = block_max(mx, sh);
+    double bm = __longlong_as_double((long long)block_max_bits(mx));
     double bs = block_sum(r2, sh);
     if (threadIdx.x == 0) {
         pt->a[blockIdx.x] = bm;
@@ -137,15 +138,16 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 6) cg_update_kernel(Grid g, dou
     if (stopped(sc)) return;
     __shared__ double sh[BLOCK_THREADS / 32];
     const double alpha = sc->alpha;
-    double mx = 0.0, r2 = 0.0;
+    unsigned long long mx = 0;
+    double r2 = 0.0;
     for_each_cell(g, [&](int i, int j, int k, long long c) {
         x[c] = fma(alpha, __ldg(s + c), x[c]);
         double rv = fma(-alpha, __ldg(z + c), r[c]);
         r[c] = rv;
-        mx = fmax(mx, fabs(rv));
+        mx = max(mx, abs_bits(rv));
         r2 = fma(rv, rv, r2);
     });
-    double bm = block_max(mx, sh);
+    double bm = __longlong_as_double((long long)block_max_bits(mx));
     double bs = block_sum(r2, sh);
     if (threadIdx.x == 0) {
         pt->b[blockIdx.x] = bm;
@@ -189,7 +191,8 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 6) true_residual_kernel(Grid g,
                                                                       const double *__restrict__ prev, Scalars *sc,
                                                                       Partials *pt) {
     __shared__ double sh[BLOCK_THREADS / 32];
-    double mx = 0.0, r2 = 0.0, b2 = 0.0;
+    unsigned long long mx = 0;
+    double r2 = 0.0, b2 = 0.0;
     const long long sy = g.nx, sz = (long long)g.nx * g.ny;
     auto X = [&](long long c) { return prev ? __ldg(x + c) + __ldg(prev + c) : __ldg(x + c); };
     for_each_cell(g, [&](int i, int j, int k, long long c) {
@@ -204,7 +207,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 6) true_residual_kernel(Grid g,
         }
         // rows off the unknowns are identically 0 (diag and couplings 0, b 0)
         const double rv = __ldg(b + c) - acc;
-        mx = fmax(mx, fabs(rv));
+        mx = max(mx, abs_bits(rv));
         r2 = fma(rv, rv, r2);
         double b0 = __ldg(b + c);
         if (prev) {
@@ -221,7 +224,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 6) true_residual_kernel(Grid g,
         }
         b2 = fma(b0, b0, b2);
     });
-    double bm = block_max(mx, sh);
+    double bm = __longlong_as_double((long long)block_max_bits(mx));
     double bs = block_sum(r2, sh);
     double bb = block_sum(b2, sh);
     if (threadIdx.x == 0) {

@@ -46,8 +46,6 @@ struct CgPersistentArgs {
 namespace cgp {
 
 constexpr int kPolls = 1 << 22;  // about two seconds
-constexpr int kPad = 288;        // 256 values, 4 apart per warp's 32: the tree's reads hit all banks
-
 // Rows of the matrix-free operator: thread t of virtual block vb has the
 // cells of tiles vb, vb + nb, ..., tz planes each, as for_each_cell walks them.
 struct GridRows {
@@ -121,37 +119,6 @@ struct CsrRows {
     }
 };
 
-// |r|'s bit pattern, 0 for a NaN (which fmax ignores)
-__device__ __forceinline__ unsigned long long abs_bits(double r) {
-    const unsigned long long b = (unsigned long long)__double_as_longlong(r) & 0x7fffffffffffffffull;
-    return b > 0x7ff0000000000000ull ? 0ull : b;
-}
-
-__device__ __forceinline__ unsigned long long warp_max_bits(unsigned long long b) {
-    const unsigned hi = (unsigned)(b >> 32), mh = __reduce_max_sync(0xffffffffu, hi);
-    const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? (unsigned)b : 0u);
-    return (unsigned long long)mh << 32 | ml;
-}
-
-// block_sum's tree over 256 padded values, by one warp; result in lane 0.
-// Lane 4w + q holds the values q, q + 4, ... of warp w's 32.
-__device__ __forceinline__ double tree256(const double *v) {
-    const int lane = threadIdx.x & 31;
-    const double *p = v + (lane >> 2) * 36 + (lane & 3);
-    double a[4];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) a[k] = p[4 * k] + p[4 * k + 16];
-    double s = (a[0] + a[2]) + (a[1] + a[3]);
-    s += __shfl_down_sync(0xffffffffu, s, 2);
-    s += __shfl_down_sync(0xffffffffu, s, 1);
-    s += __shfl_down_sync(0xffffffffu, s, 16);
-    s += __shfl_down_sync(0xffffffffu, s, 8);
-    s += __shfl_down_sync(0xffffffffu, s, 4);
-    return s;
-}
-
-__device__ __forceinline__ int pad(int t) { return t + (t >> 5) * 4; }
-
 // All blocks; false if a wait ran out. Writes before it are visible after it.
 template <bool CLUSTER> __device__ __forceinline__ bool meet(unsigned *count, unsigned &target) {
     if (CLUSTER) {
@@ -184,9 +151,9 @@ __global__ void __launch_bounds__(CLUSTER ? 1024 : 768, 1) cg_persistent_kernel(
     const int T = blockDim.x, tid = threadIdx.x, items = a.rounds * a.per_block;
     double *R = smem + tid, *S = R + items * T, *Z = S + items * T, *X = Z + items * T;
     double *red = smem + 4 * items * T;                    // padded values of every virtual block
-    double *fin = red + a.rounds * a.sub * kPad;           // the partials' 256 strided sums
-    int *meta = (int *)(fin + kPad) + tid;                 // row and neighbour bits of each item
-    unsigned *nbrs = (unsigned *)((int *)(fin + kPad) + items * T) + tid;
+    double *fin = red + a.rounds * a.sub * TREE_PAD;           // the partials' 256 strided sums
+    int *meta = (int *)(fin + TREE_PAD) + tid;                 // row and neighbour bits of each item
+    unsigned *nbrs = (unsigned *)((int *)(fin + TREE_PAD) + items * T) + tid;
     __shared__ unsigned long long smax[32];
     __shared__ int active[32];  // virtual blocks with rows: r * sub + s
     __shared__ int has[32];
@@ -241,7 +208,7 @@ __global__ void __launch_bounds__(CLUSTER ? 1024 : 768, 1) cg_persistent_kernel(
     auto partials = [&](double *out) {
         __syncthreads();
         for (int q = warp; q < n_active; q += nwarps) {
-            const double s = tree256(red + active[q] * kPad);
+            const double s = tree256(red + active[q] * TREE_PAD);
             if (lane == 0) __stcg(out + virtual_block(active[q] / a.sub, active[q] % a.sub), s);
         }
     };
@@ -250,7 +217,7 @@ __global__ void __launch_bounds__(CLUSTER ? 1024 : 768, 1) cg_persistent_kernel(
         if (tid < 256) {
             double v = 0.0;
             for (int q = tid; q < a.nb; q += 256) v += __ldcg(p + q);
-            fin[pad(tid)] = v;
+            fin[tree_at(tid)] = v;
         }
         __syncthreads();
         return warp == 0 ? tree256(fin) : 0.0;
@@ -267,7 +234,7 @@ __global__ void __launch_bounds__(CLUSTER ? 1024 : 768, 1) cg_persistent_kernel(
                 Z[m] = z;
                 dot = fma(S[m], z, dot);
             }
-            if (has[r * a.sub + sub]) red[(r * a.sub + sub) * kPad + pad(t)] = dot;
+            if (has[r * a.sub + sub]) red[(r * a.sub + sub) * TREE_PAD + tree_at(t)] = dot;
         }
         partials(a.pt->a);
         if (!(good = meet<CLUSTER>(count, target))) break;
@@ -289,7 +256,7 @@ __global__ void __launch_bounds__(CLUSTER ? 1024 : 768, 1) cg_persistent_kernel(
                 mx = b > mx ? b : mx;
                 r2 = fma(rv, rv, r2);
             }
-            if (has[r * a.sub + sub]) red[(r * a.sub + sub) * kPad + pad(t)] = r2;
+            if (has[r * a.sub + sub]) red[(r * a.sub + sub) * TREE_PAD + tree_at(t)] = r2;
         }
         mx = warp_max_bits(mx);
         if (lane == 0) smax[warp] = mx;
@@ -381,7 +348,7 @@ inline CgPersistentPlan cg_persistent_plan(int nb, int per_block, int sms) {
     p.threads = p.args.sub * BLOCK_THREADS;
     const size_t items = (size_t)p.args.rounds * per_block * p.threads;
     p.shared = items * (4 * sizeof(double) + 2 * sizeof(int)) +
-               ((size_t)p.args.rounds * p.args.sub + 1) * 288 * sizeof(double);
+               ((size_t)p.args.rounds * p.args.sub + 1) * TREE_PAD * sizeof(double);
     p.use = p.shared <= 220 * 1024 && p.args.rounds * p.args.sub <= 32 && nb <= MAX_GRID;
     return p;
 }

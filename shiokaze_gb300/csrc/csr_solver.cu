@@ -29,16 +29,17 @@ __global__ void __launch_bounds__(BLOCK_THREADS) csr_init_kernel(long long n, co
                                                                  double *r, double *s, Scalars *sc, Partials *pt,
                                                                  double residual, int max_iter) {
     __shared__ double sh[BLOCK_THREADS / 32];
-    double mx = 0.0, r2 = 0.0;
+    unsigned long long mx = 0;
+    double r2 = 0.0;
     for_each_row(n, [&](long long row) {
         const double rv = __ldg(b + row);
         x[row] = 0.0;
         r[row] = rv;
         s[row] = rv;
-        mx = fmax(mx, fabs(rv));
+        mx = max(mx, abs_bits(rv));
         r2 = fma(rv, rv, r2);
     });
-    const double bm = block_max(mx, sh);
+    const double bm = __longlong_as_double((long long)block_max_bits(mx));
     const double bs = block_sum(r2, sh);
     if (threadIdx.x == 0) {
         pt->a[blockIdx.x] = bm;
@@ -113,15 +114,16 @@ __global__ void __launch_bounds__(BLOCK_THREADS) csr_update_kernel(long long n, 
     if (stopped(sc)) return;
     __shared__ double sh[BLOCK_THREADS / 32];
     const double alpha = sc->alpha;
-    double mx = 0.0, r2 = 0.0;
+    unsigned long long mx = 0;
+    double r2 = 0.0;
     for_each_row(n, [&](long long row) {
         x[row] = fma(alpha, __ldg(s + row), x[row]);
         const double rv = fma(-alpha, __ldg(z + row), r[row]);
         r[row] = rv;
-        mx = fmax(mx, fabs(rv));
+        mx = max(mx, abs_bits(rv));
         r2 = fma(rv, rv, r2);
     });
-    const double bm = block_max(mx, sh);
+    const double bm = __longlong_as_double((long long)block_max_bits(mx));
     const double bs = block_sum(r2, sh);
     if (threadIdx.x == 0) {
         pt->b[blockIdx.x] = bm;

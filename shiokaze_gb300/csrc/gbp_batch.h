@@ -80,6 +80,7 @@ template <class T> struct BScene {
 
 struct BItem {
     int ref;     // level table index
+    int scene;   // its scene
     int tile;    // first tile (in the kernel's tiling of that level)
     int ntiles;  // consecutive tiles of the item
     int begin;   // first item of this scene in the list
@@ -108,6 +109,7 @@ constexpr int BITEM_CELLS = 512;
 // Kernels derive each item from its index, with no per-item load.
 struct BSeg {
     int ref;
+    int scene;
     int begin;
     int count;
     int m;       // tiles per item
@@ -122,7 +124,7 @@ __host__ __device__ inline BItem item_at(const BSeg *segs, int nseg, int w, int 
     const int k = w - s.begin;
     const int t = k * s.m;
     const int nt = s.ntiles - t < s.m ? s.ntiles - t : s.m;
-    return BItem{s.ref, t, nt, s.begin, s.count};
+    return BItem{s.ref, s.scene, t, nt, s.begin, s.count};
 }
 
 template <class T> struct BTail {

@@ -158,45 +158,72 @@ __device__ __forceinline__ void tile_origin(const Grid &g, long long t, int &i0,
     k0 = (int)tk * g.tz;
 }
 
-template <class T> __device__ __forceinline__ T warp_sum(T v) {
+// Block-wide reductions of BLOCK_THREADS FP64 values. A warp instruction
+// holds this GPU's FP64 pipe 16 cycles and its result takes over 100, so a
+// shuffle tree in every warp (45 instructions a block, most lanes adding
+// nothing) cost more than the pass that fed it on small grids. The values go
+// through shared memory instead and one warp adds them, eight to a lane: 12
+// instructions, in the shuffle tree's association (bitwise the same sum:
+// within a warp's 32 values halves are added, 16 apart, then 8, 4, 2, 1; then
+// the 8 warps' sums 4, 2, 1 apart). Maxima of magnitudes run on bit patterns, with
+// integer instructions alone.
+
+// where thread t's value goes: 4 apart per warp's 32, so that the lanes of
+// tree256 read different banks
+constexpr int TREE_PAD = 288;
+__device__ __forceinline__ int tree_at(int t) { return t + (t >> 5) * 4; }
+
+// The sum of 256 values placed by tree_at, by one warp; result in lane 0.
+// Lane 4w + q adds the values q, q + 4, ... of warp w's 32.
+__device__ __forceinline__ double tree256(const double *v) {
+    const int lane = threadIdx.x & 31;
+    const double *p = v + (lane >> 2) * 36 + (lane & 3);
+    double a[4];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    return v;
+    for (int k = 0; k < 4; ++k) a[k] = p[4 * k] + p[4 * k + 16];
+    double s = (a[0] + a[2]) + (a[1] + a[3]);
+    s += __shfl_down_sync(0xffffffffu, s, 2);
+    s += __shfl_down_sync(0xffffffffu, s, 1);
+    s += __shfl_down_sync(0xffffffffu, s, 16);
+    s += __shfl_down_sync(0xffffffffu, s, 8);
+    s += __shfl_down_sync(0xffffffffu, s, 4);
+    return s;
 }
 
-template <class T> __device__ __forceinline__ T warp_max(T v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_down_sync(0xffffffffu, v, o));
-    return v;
+// |x|'s bit pattern (ordered as |x| is), 0 for a NaN, which fmax ignores
+__device__ __forceinline__ unsigned long long abs_bits(double x) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(x) & 0x7fffffffffffffffull;
+    return b > 0x7ff0000000000000ull ? 0ull : b;
+}
+
+__device__ __forceinline__ unsigned long long warp_max_bits(unsigned long long b) {
+    const unsigned hi = (unsigned)(b >> 32), mh = __reduce_max_sync(0xffffffffu, hi);
+    const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? (unsigned)b : 0u);
+    return (unsigned long long)mh << 32 | ml;
 }
 
 // Block-wide sum in a fixed order; result valid in thread 0.
-template <class T> __device__ __forceinline__ T block_sum(T v, T *sh) {
-    v = warp_sum(v);
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+__device__ __forceinline__ double block_sum(double v, double *) {
+    __shared__ double vals[TREE_PAD];
     __syncthreads();
-    if (lane == 0) sh[wid] = v;
+    vals[tree_at(threadIdx.x)] = v;
     __syncthreads();
-    T r = 0;
-    if (wid == 0) {
-        r = lane < (int)(blockDim.x >> 5) ? sh[lane] : T(0);
-        r = warp_sum(r);
-    }
-    return r;
+    return threadIdx.x < 32 ? tree256(vals) : 0.0;
 }
 
-template <class T> __device__ __forceinline__ T block_max(T v, T *sh) {
-    v = warp_max(v);
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+// Block-wide maximum of abs_bits patterns; result valid in warp 0.
+__device__ __forceinline__ unsigned long long block_max_bits(unsigned long long b) {
+    __shared__ unsigned long long maxs[BLOCK_THREADS / 32];
+    b = warp_max_bits(b);
     __syncthreads();
-    if (lane == 0) sh[wid] = v;
+    if ((threadIdx.x & 31) == 0) maxs[threadIdx.x >> 5] = b;
     __syncthreads();
-    T r = 0;
-    if (wid == 0) {
-        r = lane < (int)(blockDim.x >> 5) ? sh[lane] : T(0);
-        r = warp_max(r);
-    }
-    return r;
+    return threadIdx.x < 32 ? warp_max_bits(threadIdx.x < BLOCK_THREADS / 32 ? maxs[threadIdx.x] : 0ull) : 0ull;
+}
+
+// Block-wide maximum of |v|, NaN ignored; result valid in warp 0.
+__device__ __forceinline__ double block_max(double v, double *) {
+    return __longlong_as_double((long long)block_max_bits(abs_bits(v)));
 }
 
 // Publishes this block's partial(s) and returns true in every thread of the
@@ -223,9 +250,9 @@ __device__ __forceinline__ double reduce_partials_sum(const double *partial, int
 }
 
 __device__ __forceinline__ double reduce_partials_max(const double *partial, int n, double *sh) {
-    double v = 0.0;
-    for (int t = threadIdx.x; t < n; t += blockDim.x) v = fmax(v, __ldcg(partial + t));
-    return block_max(v, sh);
+    unsigned long long v = 0;
+    for (int t = threadIdx.x; t < n; t += blockDim.x) v = max(v, abs_bits(__ldcg(partial + t)));
+    return __longlong_as_double((long long)block_max_bits(v));
 }
 
 #endif  // __CUDACC__

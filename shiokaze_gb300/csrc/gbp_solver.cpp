@@ -426,7 +426,7 @@ template <class T> void Solver::add_to_plan(BatchPlan<T> &plan, const gbp_params
         auto add = [&](std::vector<BSeg> &list, int &items, long long tiles, long long cells_per_tile) {
             const int m = (int)std::max(1LL, BITEM_CELLS / cells_per_tile);
             const int count = (int)((tiles + m - 1) / m);
-            list.push_back(BSeg{base + l, items, count, m, (int)tiles});
+            list.push_back(BSeg{base + l, s, items, count, m, (int)tiles});
             items += count;
         };
         add(plan.pair[l], plan.n_pair[l], pair_tiles(F.g), 64LL * TILE_Y * F.g.tz);
