@@ -950,43 +950,39 @@ __global__ void __launch_bounds__(BLOCK_THREADS, OCC)
 
 // ---- coarse levels in two cooperative launches -------------------------------------
 
-// Grid-wide barrier of a cooperative launch (every block resident): arrivals
-// counted on cnt->bar_count, release by a bump of cnt->bar_gen, which each
-// block reads before it arrives. The wait is bounded (about a second); a
-// block whose wait runs out records cnt->bar_err and leaves the kernel, the
-// others run out the same way, and the host reports the error.
+// Grid-wide barrier of a cooperative launch (every block resident): each
+// block adds 1 to cnt->bar_count, never reset within a solve, and waits until
+// the count reaches the next multiple of the grid (one atomic and polls of the
+// same word; a reset and a separate generation word took two more trips to L2,
+// and a sleep between polls another 0.1 us: the two cooperative kernels went
+// from 50 to 42 us an iteration at 128^3, 155 to 123 us at 256^3). The wait is bounded (about a
+// second); a block whose wait runs out records cnt->bar_err and leaves the
+// kernel, the others run out the same way, and the host reports the error.
 __device__ __forceinline__ bool grid_barrier(BatchCounters *cnt) {
-    __shared__ int ok;
     __syncthreads();
+    int good = 1;
     if (threadIdx.x == 0) {
-        volatile unsigned *gen = &cnt->bar_gen;
-        const unsigned g = *gen;
-        __threadfence();
-        int good = 1;
-        const int limit = cnt->test_polls > 0 ? cnt->test_polls : (1 << 24);
         if (cnt->test_what == 1 && (int)blockIdx.x == cnt->test_block) {
             // test hook: this block never arrives (as if it had stopped);
             // the others' waits run out
             good = 0;
-        } else if (atomicAdd(&cnt->bar_count, 1u) == gridDim.x - 1) {
-            cnt->bar_count = 0;
-            __threadfence();
-            atomicAdd(&cnt->bar_gen, 1u);
         } else {
-            for (int it = 0; *gen == g; ++it) {
+            unsigned seen;
+            asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(seen) : "l"(&cnt->bar_count) : "memory");
+            const unsigned target = (seen / gridDim.x + 1) * gridDim.x;
+            const int limit = cnt->test_polls > 0 ? cnt->test_polls : (1 << 22);
+            ++seen;
+            for (int it = 0; seen < target; ++it) {
                 if (it > limit) {
                     good = 0;
                     atomicExch(&cnt->bar_err, 1);
                     break;
                 }
-                __nanosleep(64);
+                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(&cnt->bar_count) : "memory");
             }
         }
-        __threadfence();
-        ok = good;
     }
-    __syncthreads();
-    return ok != 0;
+    return __syncthreads_and(good) != 0;
 }
 
 // Levels first..last top-down: presmooth, extra sweeps, restriction. The
@@ -1239,57 +1235,152 @@ template <class T> struct SLevel {
 };
 
 // Neighbour sum of cell (i, j, k) = c, in the order -x, +x, -y, +y, -z,
-// +z; xat(m, i', j', k') is the value at neighbour m = (i', j', k').
+// +z; xat(m, i', j', k') is the value at neighbour m = (i', j', k'). Every
+// load is issued before the sum.
 template <class T, class X>
 __device__ __forceinline__ T snb(const SLevel<T> &L, int i, int j, int k, int c, X xat) {
     const int sy = L.nx, sz = L.nx * L.ny;
+    const bool on[6] = {i > 0, i + 1 < L.nx, j > 0, j + 1 < L.ny, L.dim == 3 && k > 0, L.dim == 3 && k + 1 < L.nz};
+    T w[6], v[6];
+    w[0] = on[0] ? L.cx[c - 1] : T(0);
+    v[0] = on[0] ? xat(c - 1, i - 1, j, k) : T(0);
+    w[1] = on[1] ? L.cx[c] : T(0);
+    v[1] = on[1] ? xat(c + 1, i + 1, j, k) : T(0);
+    w[2] = on[2] ? L.cy[c - sy] : T(0);
+    v[2] = on[2] ? xat(c - sy, i, j - 1, k) : T(0);
+    w[3] = on[3] ? L.cy[c] : T(0);
+    v[3] = on[3] ? xat(c + sy, i, j + 1, k) : T(0);
+    w[4] = on[4] ? L.cz[c - sz] : T(0);
+    v[4] = on[4] ? xat(c - sz, i, j, k - 1) : T(0);
+    w[5] = on[5] ? L.cz[c] : T(0);
+    v[5] = on[5] ? xat(c + sz, i, j, k + 1) : T(0);
     T s = T(0);
-    if (i > 0) s += L.cx[c - 1] * xat(c - 1, i - 1, j, k);
-    if (i + 1 < L.nx) s += L.cx[c] * xat(c + 1, i + 1, j, k);
-    if (j > 0) s += L.cy[c - sy] * xat(c - sy, i, j - 1, k);
-    if (j + 1 < L.ny) s += L.cy[c] * xat(c + sy, i, j + 1, k);
-    if (L.dim == 3) {
-        if (k > 0) s += L.cz[c - sz] * xat(c - sz, i, j, k - 1);
-        if (k + 1 < L.nz) s += L.cz[c] * xat(c + sz, i, j, k + 1);
-    }
+#pragma unroll
+    for (int n = 0; n < 6; ++n)
+        if (on[n]) s = fmadd(s, w[n], v[n]);
     return s;
 }
 
 // Thread mapping of the tail: pair slots (2 ip, j, k), ip < hx. A pass that
 // updates one colour gives each thread the slot's cell of that colour
 // (i = 2 ip + ((j + k + color) & 1)), so no thread idles on the other
-// colour; a pass over every cell gives it both cells of the slot.
+// colour; a pass over every cell gives it both cells of the slot. A thread
+// takes its slots two at a time and stores their values after computing both,
+// so that their loads overlap (a store could alias the next slot's loads).
+struct Slot {
+    int i, j, k, c;
+    bool on;
+};
+template <class T> __device__ __forceinline__ Slot slot_cell(const SLevel<T> &L, int p, int slots, int color) {
+    Slot s;
+    const int q = p < slots ? p : 0;
+    const int t = (int)fdiv((unsigned)q, L.fhx);
+    s.k = (int)fdiv((unsigned)q, L.fhxy);
+    s.j = t - s.k * L.ny;
+    s.i = 2 * (q - t * L.hx) + (color < 0 ? 0 : ((s.j + s.k + color) & 1));
+    s.on = p < slots && s.i < L.nx;
+    if (s.i >= L.nx) s.i = 0;
+    s.c = s.i + L.nx * (s.j + L.ny * s.k);
+    return s;
+}
+// x of one colour's cells = f(cell)
 template <class T, class F> __device__ __forceinline__ void s_for_color(const SLevel<T> &L, int color, F f) {
     const int slots = L.hx * L.ny * L.nz;
-    for (int p = threadIdx.x; p < slots; p += blockDim.x) {
-        const int t = (int)fdiv((unsigned)p, L.fhx), k = (int)fdiv((unsigned)p, L.fhxy);
-        const int j = t - k * L.ny;
-        const int i = 2 * (p - t * L.hx) + ((j + k + color) & 1);
-        if (i < L.nx) f(i, j, k, i + L.nx * (j + L.ny * k));
+    for (int p = threadIdx.x; p < slots; p += 2 * blockDim.x) {
+        const Slot a = slot_cell(L, p, slots, color), b = slot_cell(L, p + (int)blockDim.x, slots, color);
+        const T va = f(a.i, a.j, a.k, a.c), vb = b.on ? f(b.i, b.j, b.k, b.c) : T(0);
+        if (a.on) L.x[a.c] = va;
+        if (b.on) L.x[b.c] = vb;
     }
     __syncthreads();
 }
-template <class T, class F> __device__ __forceinline__ void s_for_cells(const SLevel<T> &L, F f) {
+// out(cell) = f(cell) for every cell
+template <class T, class F>
+__device__ __forceinline__ void s_for_cells(const SLevel<T> &L, T *out, F f) {
     const int slots = L.hx * L.ny * L.nz;
     for (int p = threadIdx.x; p < slots; p += blockDim.x) {
-        const int t = (int)fdiv((unsigned)p, L.fhx), k = (int)fdiv((unsigned)p, L.fhxy);
-        const int j = t - k * L.ny;
-        const int i = 2 * (p - t * L.hx);
-        const int c = i + L.nx * (j + L.ny * k);
-        f(i, j, k, c);
-        if (i + 1 < L.nx) f(i + 1, j, k, c + 1);
+        const Slot a = slot_cell(L, p, slots, -1);
+        const bool second = a.i + 1 < L.nx;
+        const T va = f(a.i, a.j, a.k, a.c), vb = second ? f(a.i + 1, a.j, a.k, a.c + 1) : T(0);
+        out[a.c] = va;
+        if (second) out[a.c + 1] = vb;
     }
     __syncthreads();
 }
+
+// The coarsest level of at most one warp's slots (64 cells, 4^3): its
+// coarsest_pairs_warp symmetric FP64 sweep pairs from x = 0 are a linear map
+// of b, whose matrix the solve forms once, a warp per column (unit b). Run
+// directly they were 32 half-sweeps, each a chain of seven dependent FP64
+// operations and a barrier: 10 us of a 256^3 or 32^3 iteration's 40 or 33 us
+// tail; the matrix takes 4096 FP64 products. With it and the passes below
+// the tail went from 37 to 20 us an iteration at 128^3, 40 to 22 us at 256^3.
+constexpr int TAIL_DENSE = 64;
+__device__ __forceinline__ bool tail_dense(int hx, int ny, int nz) { return hx * ny * nz <= 32; }
+template <class T>
+__global__ void __launch_bounds__(32) tail_matrix_kernel(const BTail<T> *__restrict__ tails, MgSettings ms) {
+    const BTail<T> &A = tails[blockIdx.x / TAIL_DENSE];
+    const int col = blockIdx.x % TAIL_DENSE;
+    if (A.nt <= 0) return;
+    const MgLevel<T> &G = A.lv[A.nt - 1];
+    const int nx = G.g.nx, ny = G.g.ny, nz = G.g.nz, hx = (nx + 1) / 2, n = nx * ny * nz;
+    if (!tail_dense(hx, ny, nz) || col >= n) return;
+    __shared__ double x[TAIL_DENSE + 1];
+    if (threadIdx.x == 0) x[TAIL_DENSE] = 0.0;
+    const int p = threadIdx.x, sy = nx, sz = nx * ny;
+    x[p] = 0.0;
+    x[p + 32] = 0.0;
+    __syncwarp();
+    const int t = p / hx, k = p / (hx * ny), j = t - k * ny, i0 = 2 * (p - t * hx);
+    const int order[4] = {0, 1, 1, 0};
+    // the slot's two cells: couplings and right-hand side over the diagonal,
+    // and the neighbours (one past the cells, where x stays 0, if there is
+    // none); two sums of three keep the dependent chain at four operations
+    const int step[6] = {-1, 1, -sy, sy, -sz, sz};
+    double w[2][6], b[2];
+    int nb[2][6];
+    bool have[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const int i = i0 + h, c = i + nx * (j + ny * k);
+        have[h] = p < hx * ny * nz && i < nx;
+        const bool on[6] = {i > 0, i + 1 < nx, j > 0, j + 1 < ny, G.g.dim == 3 && k > 0, G.g.dim == 3 && k + 1 < nz};
+        const T *a[6] = {G.cx + c - 1, G.cx + c, G.cy + c - sy, G.cy + c, G.cz + c - sz, G.cz + c};
+        const double inv = have[h] ? (double)G.inv[c] : 0.0;
+#pragma unroll
+        for (int q = 0; q < 6; ++q) {
+            w[h][q] = have[h] && on[q] ? (double)*a[q] * inv : 0.0;
+            nb[h][q] = have[h] && on[q] ? c + step[q] : TAIL_DENSE;
+        }
+        b[h] = c == col ? inv : 0.0;
+    }
+    auto relax = [&](auto side) {
+        constexpr int h = decltype(side)::value;
+        if (!have[h]) return;
+        const double u = fma(w[h][2], x[nb[h][2]], fma(w[h][1], x[nb[h][1]], fma(w[h][0], x[nb[h][0]], b[h])));
+        const double v = fma(w[h][5], x[nb[h][5]], fma(w[h][4], x[nb[h][4]], w[h][3] * x[nb[h][3]]));
+        x[i0 + h + nx * (j + ny * k)] = u + v;
+    };
+    for (int pr = 0; pr < ms.coarsest_pairs_warp; ++pr)
+        for (int q = 0; q < 4; ++q) {
+            if ((j + k + order[q]) & 1) relax(std::integral_constant<int, 1>{});
+            else relax(std::integral_constant<int, 0>{});
+            __syncwarp();
+        }
+    for (int r = p; r < n; r += 32) A.m64[r * TAIL_DENSE + col] = x[r];
+}
+
 // The V-cycle of the levels lv[0..nt) in one block per scene: b of lv[0]
 // in, x of lv[0] out, same smoother, transfers and coarsest solve (FP64
-// symmetric sweep pairs, with the coarsest operator and right-hand side
-// held in FP64) as the global levels. The levels (a few hundred KB at
-// most) are read and written in place in global memory, where the block's
-// L1 holds them between passes; __syncthreads orders a pass's writes
-// before the next pass's reads within the block. (A copy into shared memory
-// needs a carveout of the SM's L1 different from every other kernel's, and
-// the switch costs more than the copy saves.)
+// symmetric sweep pairs, as a matrix where tail_dense, else with the coarsest
+// operator and right-hand side held in FP64) as the global levels. The levels
+// (a few hundred KB at most) are read and written in place in global memory,
+// where the block's L1 holds them between passes; __syncthreads orders a
+// pass's writes before the next pass's reads within the block. (A copy into
+// shared memory needs a carveout of the SM's L1 different from every other
+// kernel's, and the switch costs more than the copy saves.) The block is
+// bound by latency: passes issue their loads first, and the restriction goes
+// through residuals in shared memory, a thread per fine pair.
 template <class T>
 __global__ void __launch_bounds__(MG_TAIL_THREADS) tail_kernel(const BTail<T> *__restrict__ tails,
                                                                const BScene<T> *__restrict__ scenes, int gate,
@@ -1301,49 +1392,49 @@ __global__ void __launch_bounds__(MG_TAIL_THREADS) tail_kernel(const BTail<T> *_
     if (gated(scenes[s].sc, gate)) return;
     __shared__ SLevel<T> S[MG_MAX_LEVELS];
     __shared__ double *cd[6];  // coarsest: x, b, inv, cx, cy, cz in FP64
-    if (threadIdx.x == 0) {
-        for (int l = 0; l < A.nt; ++l) {
-            const MgLevel<T> &G = A.lv[l];
-            const Grid &g = G.g;
-            SLevel<T> &L = S[l];
-            L.nx = g.nx;
-            L.ny = g.ny;
-            L.nz = g.nz;
-            L.dim = g.dim;
-            L.n = (int)g.ncell;
-            L.hx = (g.nx + 1) / 2;
-            L.fhx = make_fastdiv((unsigned)L.hx);
-            L.fhxy = make_fastdiv((unsigned)(L.hx * g.ny));
-            L.b = G.b;
-            L.x = G.x;
-            L.inv = const_cast<T *>(G.inv);
-            L.diag = const_cast<T *>(G.diag);
-            L.cx = const_cast<T *>(G.cx);
-            L.cy = const_cast<T *>(G.cy);
-            L.cz = const_cast<T *>(G.cz);  // == cy in 2D, never read there
-        }
-        for (int a = 0; a < 6; ++a) cd[a] = A.c64 + (size_t)a * MG_COARSEST_MAX;
+    __shared__ T res[MG_TAIL_BYTES_MAX / (7 * sizeof(T)) + 1];  // a level's residuals
+    __shared__ double bc[TAIL_DENSE];
+    if (threadIdx.x < A.nt) {
+        const MgLevel<T> &G = A.lv[threadIdx.x];
+        const Grid &g = G.g;
+        SLevel<T> &L = S[threadIdx.x];
+        L.nx = g.nx;
+        L.ny = g.ny;
+        L.nz = g.nz;
+        L.dim = g.dim;
+        L.n = (int)g.ncell;
+        L.hx = (g.nx + 1) / 2;
+        L.fhx = make_fastdiv((unsigned)L.hx);
+        L.fhxy = make_fastdiv((unsigned)(L.hx * g.ny));
+        L.b = G.b;
+        L.x = G.x;
+        L.inv = const_cast<T *>(G.inv);
+        L.diag = const_cast<T *>(G.diag);
+        L.cx = const_cast<T *>(G.cx);
+        L.cy = const_cast<T *>(G.cy);
+        L.cz = const_cast<T *>(G.cz);  // == cy in 2D, never read there
     }
+    if (threadIdx.x < 6) cd[threadIdx.x] = A.c64 + (size_t)threadIdx.x * MG_COARSEST_MAX;
     __syncthreads();
     const T alpha = T(ms.alpha);
     for (int l = 0; l + 1 < A.nt; ++l) {
         const SLevel<T> &L = S[l];
-        s_for_cells(L, [&](int i, int j, int k, int c) {
+        s_for_cells(L, L.x, [&](int i, int j, int k, int c) {
             const T inv = L.inv[c];
-            if (((i + j + k) & 1) == 0) {
-                L.x[c] = L.b[c] * inv;
-            } else {
-                L.x[c] = (L.b[c] + snb(L, i, j, k, c, [&](int m, int, int, int) { return L.b[m] * L.inv[m]; })) *
-                         inv;
-            }
+            if (((i + j + k) & 1) == 0) return L.b[c] * inv;
+            return (L.b[c] + snb(L, i, j, k, c, [&](int m, int, int, int) { return L.b[m] * L.inv[m]; })) * inv;
         });
         for (int sw = 1; sw < ms.smooth; ++sw)
             for (int color = 0; color < 2; ++color)
                 s_for_color(L, color, [&](int i, int j, int k, int c) {
-                    L.x[c] = (L.b[c] + snb(L, i, j, k, c, [&](int m, int, int, int) { return L.x[m]; })) * L.inv[c];
+                    return (L.b[c] + snb(L, i, j, k, c, [&](int m, int, int, int) { return L.x[m]; })) * L.inv[c];
                 });
         const SLevel<T> &C = S[l + 1];
-        s_for_cells(C, [&](int I, int J, int K, int cc) {
+        s_for_cells(L, res, [&](int i, int j, int k, int c) {
+            return resid(L.b[c], L.diag[c], L.x[c],
+                         snb(L, i, j, k, c, [&](int m, int, int, int) { return L.x[m]; }));
+        });
+        s_for_cells(C, C.b, [&](int I, int J, int K, int) {
             T sum = T(0);
             const int kmax = L.dim == 3 ? 2 : 1;
             for (int c2 = 0; c2 < kmax; ++c2)
@@ -1351,79 +1442,91 @@ __global__ void __launch_bounds__(MG_TAIL_THREADS) tail_kernel(const BTail<T> *_
                     for (int a2 = 0; a2 < 2; ++a2) {
                         const int i = 2 * I + a2, j = 2 * J + b2, k = 2 * K + c2;
                         if (i >= L.nx || j >= L.ny || k >= L.nz) continue;
-                        const int f = i + L.nx * (j + L.ny * k);
-                        sum += L.b[f] -
-                               (L.diag[f] * L.x[f] - snb(L, i, j, k, f, [&](int m, int, int, int) { return L.x[m]; }));
+                        sum += res[i + L.nx * (j + L.ny * k)];
                     }
-            C.b[cc] = sum;
+            return sum;
         });
     }
     {
         const SLevel<T> &L = S[A.nt - 1];
-        double *xc = cd[0], *bd = cd[1], *ivd = cd[2], *cxd = cd[3], *cyd = cd[4], *czd = cd[5];
-        for (int c = threadIdx.x; c < L.n; c += blockDim.x) {
-            xc[c] = 0.0;
-            bd[c] = (double)L.b[c];
-            ivd[c] = (double)L.inv[c];
-            cxd[c] = (double)L.cx[c];
-            cyd[c] = (double)L.cy[c];
-            czd[c] = (double)L.cz[c];
-        }
-        __syncthreads();
-        const int sy = L.nx, sz = L.nx * L.ny;
-        auto relax = [&](int i, int j, int k, int c) {
-            double acc = 0.0;
-            if (i > 0) acc += cxd[c - 1] * xc[c - 1];
-            if (i + 1 < L.nx) acc += cxd[c] * xc[c + 1];
-            if (j > 0) acc += cyd[c - sy] * xc[c - sy];
-            if (j + 1 < L.ny) acc += cyd[c] * xc[c + sy];
-            if (L.dim == 3) {
-                if (k > 0) acc += czd[c - sz] * xc[c - sz];
-                if (k + 1 < L.nz) acc += czd[c] * xc[c + sz];
-            }
-            xc[c] = (bd[c] + acc) * ivd[c];
-        };
-        const int order[4] = {0, 1, 1, 0};
         const int slots = L.hx * L.ny * L.nz;
-        if (slots <= 32) {
-            // a coarsest level of one warp's slots (4^3 and below): the
-            // warp sweeps it alone, with warp barriers between half-sweeps,
-            // so it can afford more sweep pairs
-            if (threadIdx.x < 32) {
-                const int p = threadIdx.x;
-                const int t = (int)fdiv((unsigned)p, L.fhx), k = (int)fdiv((unsigned)p, L.fhxy);
-                const int j = t - k * L.ny;
-                for (int pr = 0; pr < ms.coarsest_pairs_warp; ++pr)
-                    for (int q = 0; q < 4; ++q) {
-                        const int i = 2 * (p - t * L.hx) + ((j + k + order[q]) & 1);
-                        if (p < slots && i < L.nx) relax(i, j, k, i + L.nx * (j + L.ny * k));
-                        __syncwarp();
-                    }
+        if (tail_dense(L.hx, L.ny, L.nz)) {
+            // x = M b, four threads a row
+            if (threadIdx.x < 4 * TAIL_DENSE) {
+                const int r = threadIdx.x >> 2, q = threadIdx.x & 3;
+                double m[TAIL_DENSE / 4];
+#pragma unroll
+                for (int e = 0; e < TAIL_DENSE / 4; ++e)
+                    m[e] = r < L.n && 4 * e + q < L.n ? __ldcg(A.m64 + r * TAIL_DENSE + 4 * e + q) : 0.0;
+                if (threadIdx.x < TAIL_DENSE) bc[threadIdx.x] = threadIdx.x < L.n ? widen(L.b[threadIdx.x]) : 0.0;
+                asm volatile("bar.sync 1, %0;" ::"n"(4 * TAIL_DENSE) : "memory");
+                double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
+#pragma unroll
+                for (int e = 0; e < TAIL_DENSE / 4; e += 4) {
+                    a0 = fma(m[e], bc[4 * e + q], a0);
+                    a1 = fma(m[e + 1], bc[4 * e + 4 + q], a1);
+                    a2 = fma(m[e + 2], bc[4 * e + 8 + q], a2);
+                    a3 = fma(m[e + 3], bc[4 * e + 12 + q], a3);
+                }
+                double v = (a0 + a1) + (a2 + a3);
+                v += __shfl_xor_sync(0xffffffffu, v, 1);
+                v += __shfl_xor_sync(0xffffffffu, v, 2);
+                if (q == 0 && r < L.n) L.x[r] = narrow_to<T>(v);
             }
             __syncthreads();
         } else {
+            double *xc = cd[0], *bd = cd[1], *ivd = cd[2], *cxd = cd[3], *cyd = cd[4], *czd = cd[5];
+            for (int c = threadIdx.x; c < L.n; c += blockDim.x) {
+                xc[c] = 0.0;
+                bd[c] = (double)L.b[c];
+                ivd[c] = (double)L.inv[c];
+                cxd[c] = (double)L.cx[c];
+                cyd[c] = (double)L.cy[c];
+                czd[c] = (double)L.cz[c];
+            }
+            __syncthreads();
+            const int sy = L.nx, sz = L.nx * L.ny;
+            const int order[4] = {0, 1, 1, 0};
             for (int p = 0; p < ms.coarsest_pairs; ++p)
-                for (int q = 0; q < 4; ++q) s_for_color(L, order[q], relax);
+                for (int q = 0; q < 4; ++q) {
+                    for (int e = threadIdx.x; e < slots; e += blockDim.x) {
+                        const Slot a = slot_cell(L, e, slots, order[q]);
+                        if (!a.on) continue;
+                        const int i = a.i, j = a.j, k = a.k, c = a.c;
+                        double acc = 0.0;
+                        if (i > 0) acc += cxd[c - 1] * xc[c - 1];
+                        if (i + 1 < L.nx) acc += cxd[c] * xc[c + 1];
+                        if (j > 0) acc += cyd[c - sy] * xc[c - sy];
+                        if (j + 1 < L.ny) acc += cyd[c] * xc[c + sy];
+                        if (L.dim == 3) {
+                            if (k > 0) acc += czd[c - sz] * xc[c - sz];
+                            if (k + 1 < L.nz) acc += czd[c] * xc[c + sz];
+                        }
+                        xc[c] = (bd[c] + acc) * ivd[c];
+                    }
+                    __syncthreads();
+                }
+            for (int c = threadIdx.x; c < L.n; c += blockDim.x) L.x[c] = T(xc[c]);
+            __syncthreads();
         }
-        for (int c = threadIdx.x; c < L.n; c += blockDim.x) L.x[c] = T(xc[c]);
-        __syncthreads();
     }
     for (int l = A.nt - 2; l >= 0; --l) {
         const SLevel<T> &L = S[l];
         const SLevel<T> &C = S[l + 1];
         const bool d3 = L.dim == 3;
         s_for_color(L, 1, [&](int i, int j, int k, int c) {
-            L.x[c] = (L.b[c] + snb(L, i, j, k, c, [&](int m, int mi, int mj, int mk) {
-                         return L.x[m] + alpha * C.x[(mi >> 1) + C.nx * ((mj >> 1) + C.ny * (d3 ? (mk >> 1) : 0))];
-                     })) * L.inv[c];
+            return (L.b[c] + snb(L, i, j, k, c, [&](int m, int mi, int mj, int mk) {
+                        return prolong(L.x[m], alpha,
+                                       C.x[(mi >> 1) + C.nx * ((mj >> 1) + C.ny * (d3 ? (mk >> 1) : 0))]);
+                    })) * L.inv[c];
         });
         for (int sw = 1; sw < ms.smooth; ++sw)
             for (int color = 0; color < 2; ++color)
                 s_for_color(L, color, [&](int i, int j, int k, int c) {
-                    L.x[c] = (L.b[c] + snb(L, i, j, k, c, [&](int m, int, int, int) { return L.x[m]; })) * L.inv[c];
+                    return (L.b[c] + snb(L, i, j, k, c, [&](int m, int, int, int) { return L.x[m]; })) * L.inv[c];
                 });
         s_for_color(L, 0, [&](int i, int j, int k, int c) {
-            L.x[c] = (L.b[c] + snb(L, i, j, k, c, [&](int m, int, int, int) { return L.x[m]; })) * L.inv[c];
+            return (L.b[c] + snb(L, i, j, k, c, [&](int m, int, int, int) { return L.x[m]; })) * L.inv[c];
         });
     }
 }
@@ -2323,6 +2426,10 @@ cudaError_t b_tail(const BLaunch &L, const BTail<T> *tails, int nscenes, const B
     tail_kernel<T><<<nscenes, MG_TAIL_THREADS, 0, L.stream>>>(tails, scenes, L.gate, ms, L.cnt);
     return cudaGetLastError();
 }
+template <class T> cudaError_t b_tail_matrix(cudaStream_t st, const BTail<T> *tails, int nscenes, MgSettings ms) {
+    tail_matrix_kernel<T><<<nscenes * TAIL_DENSE, 32, 0, st>>>(tails, ms);
+    return cudaGetLastError();
+}
 template <class T>
 cudaError_t b_coarse_descend(const BLaunch &L, const BLevel<T> *levels, const CoarseLists &cl,
                              const BScene<T> *scenes, MgSettings ms) {
@@ -2454,6 +2561,7 @@ cudaError_t b_refine_residual(const BLaunch &L, const BLevel<T> *levels, const B
     template cudaError_t b_red_dot<T>(const BLaunch &, const BLevel<T> *, const BSeg *, int, int,                   \
                                       const BScene<T> *, double *);                                                  \
     template cudaError_t b_tail<T>(const BLaunch &, const BTail<T> *, int, const BScene<T> *, MgSettings);            \
+    template cudaError_t b_tail_matrix<T>(cudaStream_t, const BTail<T> *, int, MgSettings);                           \
     template cudaError_t b_coarse_descend<T>(const BLaunch &, const BLevel<T> *, const CoarseLists &,                 \
                                              const BScene<T> *, MgSettings);                                         \
     template cudaError_t b_coarse_ascend<T>(const BLaunch &, const BLevel<T> *, const CoarseLists &,                  \

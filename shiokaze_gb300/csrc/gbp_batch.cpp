@@ -185,10 +185,13 @@ template <class T> int BatchRunner::build(const BatchPlan<T> &plan, int grid_blo
     {
         // FP64 scratch of each scene's coarsest level, then the tail table
         void *d;
-        const size_t per = 6 * (size_t)MG_COARSEST_MAX;
+        const size_t per = 6 * (size_t)MG_COARSEST_MAX + TAIL_MATRIX;
         if ((rc = upload(nullptr, sizeof(double) * per * std::max<size_t>(1, plan.tails.size()), &d))) return rc;
         std::vector<BTail<T>> tails = plan.tails;
-        for (size_t s = 0; s < tails.size(); ++s) tails[s].c64 = static_cast<double *>(d) + s * per;
+        for (size_t s = 0; s < tails.size(); ++s) {
+            tails[s].c64 = static_cast<double *>(d) + s * per;
+            tails[s].m64 = tails[s].c64 + 6 * (size_t)MG_COARSEST_MAX;
+        }
         if ((rc = upload(tails.data(), tails.size() * sizeof(BTail<T>), &d_tails_))) return rc;
     }
     size_t max_items = (size_t)plan.n_fine_pairs;
@@ -407,7 +410,9 @@ template <class T> int BatchRunner::tune_occupancy(cudaStream_t st, const std::s
                 return e;
             };
             float t[3] = {0.f, 0.f, 0.f};
-            err = run();
+            // the barriers count in multiples of the grid
+            err = cudaMemsetAsync(&d_counters_->bar_count, 0, sizeof(unsigned), st);
+            if (err == cudaSuccess) err = run();
             for (int r = 0; r < 3 && err == cudaSuccess; ++r) {
                 err = cudaEventRecord(e0, st);
                 if (err == cudaSuccess) err = run();
@@ -560,6 +565,10 @@ template <class T> int BatchRunner::solve(const gbp_params &p, cudaStream_t st, 
                                   d_fine_pairs_, s_fine_pairs_, n_fine_pairs_, sc, d_part_, 1, p.residual, p.max_iterations, inner_rel_, kInnerMax,
                                   d_counters_));
     *launches += 1;
+    if (tail_bytes_ > 0) {
+        RUN_CUDA(b_tail_matrix<T>(st, static_cast<const BTail<T> *>(d_tails_), nscenes_, settings_of(p)));
+        *launches += 1;
+    }
     const long long key = ((long long)(p.mg_smooth > 0 ? p.mg_smooth : 1) << 40) ^
                           (long long)(p.residual * 1e15) ^ ((long long)p.max_iterations << 8) ^
                           (long long)(inner_rel_ * 1e12);

@@ -133,6 +133,9 @@ template <class T> struct BTail {
     // the coarsest level in FP64 (x, b, inv, cx, cy, cz; MG_COARSEST_MAX
     // each), scratch of the batch runner
     double *c64;
+    // the coarsest solve as a matrix, 64 x 64 (a coarsest level of at most 64
+    // cells; formed by b_tail_matrix at the start of a solve)
+    double *m64;
 };
 
 // Tilings: pair tiles (64 x 8 x tz) for the red-black kernels, cell tiles
@@ -143,8 +146,7 @@ inline long long cell_tiles(const Grid &g) { return g.ntiles; }
 struct BatchCounters {
     int remaining;        // scenes not done
     int refine;           // scenes whose inner solve ended, awaiting refinement
-    unsigned bar_count;   // grid barrier of the coarse-level kernels: arrivals
-    unsigned bar_gen;     // ... and generation
+    unsigned bar_count;   // grid barriers of the coarse-level kernels: arrivals, a multiple of the grid between launches
     int bar_err;          // a barrier wait ran out (the solve is abandoned)
     // test hook (gbp_debug_fail_wait), 0 in every ordinary solve: block
     // test_block of the kernels named by test_what (1: the cooperative
@@ -306,6 +308,9 @@ cudaError_t b_red_dot(const BLaunch &L, const BLevel<T> *levels, const BSeg *seg
                       double *part);
 template <class T>
 cudaError_t b_tail(const BLaunch &L, const BTail<T> *tails, int nscenes, const BScene<T> *scenes, MgSettings ms);
+// The coarsest solves' matrices (BTail::m64), once per solve.
+template <class T> cudaError_t b_tail_matrix(cudaStream_t st, const BTail<T> *tails, int nscenes, MgSettings ms);
+constexpr int TAIL_MATRIX = 64 * 64;
 // The coarse levels' descent (presmooth, sweeps, restrict per level) and
 // ascent (post_black, sweeps, red sweep per level) as cooperative launches
 // with grid barriers between passes; L.blocks must not exceed
