@@ -20,12 +20,11 @@ struct AdvectWork {
     gba::MinMax *vmm = nullptr;  // limiter record per face
     float *q0 = nullptr;   // forward scalar
     gba::MinMax *qmm = nullptr;  // limiter record per cell
-    int *flag = nullptr;         // the solid constraint's levelset_exist flag
-    // extrapolation: the second value and mask buffers of a dilation round,
-    // and the counter of cells it activated
+    unsigned *flag = nullptr;    // the solid constraint's face count and levelset_exist flag
+    // extrapolation: a stamp byte per cell (padded), and the counter of cells
+    // it activated
     long long ext_cap = 0;
-    float *ext_a = nullptr;
-    unsigned char *ext_m = nullptr;
+    unsigned char *ext_stamp = nullptr;
     unsigned long long *ext_count = nullptr;
 };
 
@@ -69,9 +68,8 @@ cudaError_t constrain_run(AdvectWork &w, const ConstrainArgs &a, cudaStream_t st
 // src/array/dilate3.h:43-95): `count` rounds, each activating every
 // inactive in-bounds 6-neighbour of an active cell with the float mean of
 // its active neighbours, summed in the order +x, -x, +y, -y, -z, +z, all
-// computed from the state before the round. One launch per round into the
-// second buffers (held in w), then the roles swap; the result ends in a and
-// m. When activated_host is not null, the number of cells activated is
+// computed from the state before the round. One launch per round, in place
+// on a, with the cells' rounds in stamp bytes (held in w). When activated_host is not null, the number of cells activated is
 // copied there (valid once the stream is synchronised).
 cudaError_t extrapolate_run(AdvectWork &w, int W, int H, int D, float *a, unsigned char *m, int count,
                             cudaStream_t stream, long long *launches, unsigned long long *activated_host);

@@ -754,6 +754,82 @@ GBA_HD void derivative(const Shape &s, const double p[3], const float *a, float 
     }
 }
 
+// The constraint's positions are whole and half cells: every weight is 0,
+// 0.5 or 1 and every product of weights a power of two (or 0), so a value
+// times it is exact and the float accumulations of interp and derivative
+// round as plain float additions (the double sum of two floats, rounded to
+// float, is their float sum: 53 >= 2*24 + 2 bits). The whole solid branch then
+// needs double precision for its last dozen operations only. Values within
+// 2^26 of the float range's lower end would lose bits in the products; they
+// keep the double forms (half_exact).
+struct HalfAxis {
+    int i;
+    float w0, w1;
+};
+
+// the cell and weights of position p2/2, clamped as Corner is
+GBA_HD HalfAxis half_axis(int p2, int w) {
+    p2 = p2 < 0 ? 0 : (p2 > 2 * (w - 1) ? 2 * (w - 1) : p2);
+    HalfAxis a;
+    a.i = (p2 >> 1) < w - 2 ? (p2 >> 1) : w - 2;
+    a.w1 = 0.5f * (float)(p2 - 2 * a.i);
+    a.w0 = 1.0f - a.w1;
+    return a;
+}
+
+struct HalfCorner {
+    HalfAxis x, y, z;
+    float v[8];
+};
+
+GBA_HD HalfCorner half_corner(const Shape &s, const int p2[3], const float *a) {
+    HalfCorner h{half_axis(p2[0], s.w), half_axis(p2[1], s.h), half_axis(p2[2], s.d), {}};
+    const float *b = a + at(s, h.x.i, h.y.i, h.z.i);
+    const long long sy = s.w, sz = (long long)s.w * s.h;
+#pragma unroll
+    for (int n = 0; n < 8; ++n) h.v[n] = b[(n & 1) + ((n & 2) ? sy : 0) + ((n & 4) ? sz : 0)];
+    return h;
+}
+
+GBA_HD bool half_exact(const HalfCorner &h) {
+    bool ok = true;
+#pragma unroll
+    for (int n = 0; n < 8; ++n) ok = ok && (h.v[n] == 0.0f || fabsf(h.v[n]) >= 0x1p-100f || h.v[n] != h.v[n]);
+    return ok;
+}
+
+// interp at a half position
+GBA_HD float interp_half(const Shape &s, const int p2[3], const float *a) {
+    const HalfCorner h = half_corner(s, p2, a);
+    if (!half_exact(h)) return interp(s, 0.5 * p2[0], 0.5 * p2[1], 0.5 * p2[2], [a](long long n) { return a[n]; });
+    float value = 0.0f;
+#pragma unroll
+    for (int n = 0; n < 8; ++n) {
+        const float c = ((n & 4) ? h.z.w1 : h.z.w0) * ((n & 1) ? h.x.w1 : h.x.w0) * ((n & 2) ? h.y.w1 : h.y.w0);
+        if (c != 0.0f) value = value + h.v[n] * c;
+    }
+    return value;
+}
+
+// derivative at a half position
+GBA_HD void derivative_half(const Shape &s, const int p2[3], const float *a, float out[3]) {
+    const HalfCorner h = half_corner(s, p2, a);
+    if (!half_exact(h)) {
+        const double p[3] = {0.5 * p2[0], 0.5 * p2[1], 0.5 * p2[2]};
+        derivative(s, p, a, out);
+        return;
+    }
+    float r[3] = {0.0f, 0.0f, 0.0f};
+#pragma unroll
+    for (int n = 0; n < 8; ++n) {
+        const float wx = (n & 1) ? h.x.w1 : h.x.w0, wy = (n & 2) ? h.y.w1 : h.y.w0, wz = (n & 4) ? h.z.w1 : h.z.w0;
+        r[0] = r[0] + ((n & 1) ? wz * wy : -(wz * wy)) * h.v[n];
+        r[1] = r[1] + ((n & 2) ? wz * wx : -(wz * wx)) * h.v[n];
+        r[2] = r[2] + ((n & 4) ? wx * wy : -(wx * wy)) * h.v[n];
+    }
+    for (int d = 0; d < 3; ++d) out[d] = r[d];
+}
+
 struct ConstrainArgs {
     Dims g;
     const float *solid;     // nodal level set (nx+1)(ny+1)(nz+1)
@@ -766,19 +842,14 @@ struct ConstrainArgs {
 
 // compare_interp(s, p, a, 0.0) from float comparisons alone when the eight
 // corners lie clearly on one side of 0: -1 (all below) or 1 (all above),
-// else 2 (the full test decides). p2 holds twice the position: whole and
-// half nodes, as the faces' positions are. The corners and the float
+// else 2 (the full test decides), for the corners of cell (i, j, k) of the
+// nodal array; sign_corners_fast takes twice a position (whole and half nodes,
+// as the faces' positions are). The corners and the float
 // min/max/sum are compare_interp's; its range test is decided here when
 // |the corner nearest 0| >= max(2^-19 am, 2^-100), am the largest
 // magnitude, which exceeds its margin d = 2^-20 am + 1e-38 (so the double
 // test gives the same answer).
-GBA_HD int sign_corners_fast(const Shape &s, const int p2[3], const float *a) {
-    auto cell = [](int v2, int w) {
-        v2 = v2 < 0 ? 0 : (v2 > 2 * (w - 1) ? 2 * (w - 1) : v2);
-        const int c = v2 >> 1;
-        return c < w - 2 ? c : w - 2;
-    };
-    const int i = cell(p2[0], s.w), j = cell(p2[1], s.h), k = cell(p2[2], s.d);
+GBA_HD int sign_cell_fast(const Shape &s, int i, int j, int k, const float *a) {
     const long long base = at(s, i, j, k);
     const long long sy = s.w, sz = (long long)s.w * s.h;
     const long long off[8] = {0, 1, sy, sy + 1, sz, sz + 1, sz + sy, sz + sy + 1};
@@ -800,42 +871,49 @@ GBA_HD int sign_corners_fast(const Shape &s, const int p2[3], const float *a) {
     return 2;
 }
 
+GBA_HD int sign_corners_fast(const Shape &s, const int p2[3], const float *a) {
+    return sign_cell_fast(s, half_axis(p2[0], s.w).i, half_axis(p2[1], s.h).i, half_axis(p2[2], s.d).i, a);
+}
+
 // The solid branch of one face (macutility3.cpp:70-80): the saved velocity
 // interpolated at the face minus its projection on the solid's gradient
-// when that projection is negative; `in` otherwise.
-GBA_HD_OUTLINE float constrain_solid(const ConstrainArgs a, int dim, int i, int j, int k, float in, int side) {
-    const Dims &g = a.g;
-    const int ip[3] = {i, j, k};
-    const float *save[3] = {a.save, a.save + a.off1, a.save + a.off2};
-    const double p[3] = {ip[0] + 0.5 * (dim != 0), ip[1] + 0.5 * (dim != 1), ip[2] + 0.5 * (dim != 2)};
-    float val = in;
+// when that projection is negative; `in` otherwise. `side` is
+// sign_corners_fast's answer.
+GBA_HD float constrain_solid(const Dims &g, const float *solid, const float *const save[3], int dim, int i, int j,
+                             int k, float in, int side) {
+    const int p2[3] = {2 * i + (dim != 0), 2 * j + (dim != 1), 2 * k + (dim != 2)};
     const Shape ns{g.nx + 1, g.ny + 1, g.nz + 1};
-    if (side == 2) side = compare_interp(ns, p[0], p[1], p[2], a.solid, 0.0);
-    if (side == -1) {
-        float dr[3];
-        derivative(ns, p, a.solid, dr);
-        double nrm[3];
+    if (side == 2) side = interp_half(ns, p2, solid) < 0.0f ? -1 : 1;
+    if (side != -1) return in;
+    float dr[3];
+    derivative_half(ns, p2, solid, dr);
+    double nrm[3];
 #pragma unroll
-        for (int c = 0; c < 3; ++c) nrm[c] = (double)dr[c] / g.dx;
-        double n2 = 0.0;
+    for (int c = 0; c < 3; ++c) nrm[c] = g.pow2 ? (double)dr[c] * g.inv_dx : (double)dr[c] / g.dx;
+    double n2 = 0.0;
 #pragma unroll
-        for (int c = 0; c < 3; ++c) n2 += nrm[c] * nrm[c];
-        if (n2 != 0.0) {
-            // macarray_interpolator3::interpolate (macarray_interpolator3.h:49-56)
-            double uu[3];
+    for (int c = 0; c < 3; ++c) n2 += nrm[c] * nrm[c];
+    if (n2 == 0.0) return in;
+    // macarray_interpolator3::interpolate (macarray_interpolator3.h:49-56)
+    double uu[3];
 #pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                const float *sc = save[c];
-                uu[c] = interp(face_shape(g, c), p[0] - 0.5 * (c != 0), p[1] - 0.5 * (c != 1), p[2] - 0.5 * (c != 2),
-                               [sc](long long n) { return sc[n]; });
-            }
-            double dot = 0.0;
-#pragma unroll
-            for (int c = 0; c < 3; ++c) dot += uu[c] * nrm[c];
-            if (dot < 0.0) val = (float)((dim == 0 ? uu[0] : (dim == 1 ? uu[1] : uu[2])) -
-                                         (dim == 0 ? nrm[0] : (dim == 1 ? nrm[1] : nrm[2])) * dot);
-        }
+    for (int c = 0; c < 3; ++c) {
+        const int q2[3] = {p2[0] - (c != 0), p2[1] - (c != 1), p2[2] - (c != 2)};
+        uu[c] = interp_half(face_shape(g, c), q2, save[c]);
     }
+    double dot = 0.0;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) dot += uu[c] * nrm[c];
+    if (!(dot < 0.0)) return in;
+    return (float)((dim == 0 ? uu[0] : (dim == 1 ? uu[1] : uu[2])) -
+                   (dim == 0 ? nrm[0] : (dim == 1 ? nrm[1] : nrm[2])) * dot);
+}
+
+// the wall clamps of face ip of component dim (macutility3.cpp:81-84)
+GBA_HD float constrain_wall(const Dims &g, int dim, int ip, float val) {
+    const int n = dim == 0 ? g.nx : (dim == 1 ? g.ny : g.nz);
+    if (ip == 0 && val < 0.0f) val = 0.0f;
+    if (ip == n && val > 0.0f) val = 0.0f;
     return val;
 }
 
@@ -843,7 +921,9 @@ GBA_HD_OUTLINE float constrain_solid(const ConstrainArgs a, int dim, int i, int 
 // saved velocity (macutility3.cpp:68); the loop is idempotent (the solid
 // branch sets the same value from the saved velocity each time, and the
 // wall clamps are idempotent), so one pass gives its result. Faces whose
-// solid corners are all clearly positive skip the FP64 work.
+// solid corners are all clearly positive skip the solid branch. The kernels
+// take a face's steps apart (cst_scan, cst_solid, cst_apply); this is the
+// whole of them for one face, from a saved copy of the velocity.
 GBA_HD void constrain_face(const ConstrainArgs &a, int dim, unsigned f) {
     const Dims &g = a.g;
     const Shape fs = face_shape(g, dim);
@@ -857,10 +937,9 @@ GBA_HD void constrain_face(const ConstrainArgs &a, int dim, unsigned f) {
     const Shape ns{g.nx + 1, g.ny + 1, g.nz + 1};
     const int p2[3] = {2 * ip[0] + (dim != 0), 2 * ip[1] + (dim != 1), 2 * ip[2] + (dim != 2)};
     const int side = sign_corners_fast(ns, p2, a.solid);
-    if (side != 1) val = constrain_solid(a, dim, ip[0], ip[1], ip[2], in, side);
-    const int n_dim = dim == 0 ? g.nx : (dim == 1 ? g.ny : g.nz);
-    if (ip[dim] == 0 && val < 0.0f) val = 0.0f;
-    if (ip[dim] == n_dim && val > 0.0f) val = 0.0f;
+    const float *const save[3] = {a.save, a.save + a.off1, a.save + a.off2};
+    if (side != 1) val = constrain_solid(g, a.solid, save, dim, ip[0], ip[1], ip[2], in, side);
+    val = constrain_wall(g, dim, ip[dim], val);
     float *io = dim == 0 ? a.u : (dim == 1 ? a.v : a.w);
     union {
         float f;
