@@ -64,12 +64,12 @@ bool encode_map(CUtensorMap *m, const float *ptr, int nx, int ny, int nz, unsign
 }
 
 // The STAGE_MAPS maps of a fine FP32 level, or false if the level does not
-// qualify: 3D, 4-plane tiles (one tile per item), nx a multiple of 8 (rows
+// qualify: 3D, at least 2^21 cells, 4-plane tiles (one tile per item), nx a multiple of 8 (rows
 // of the level and of its coarse grid are multiples of 16 bytes, every box
 // x start a multiple of 4 floats), every array 16-byte aligned.
 bool stage_maps(const BLevel<float> &L, const BScene<float> &S, CUtensorMap *m) {
     const Grid &g = L.g, &c = L.gc;
-    if (g.dim != 3 || g.tz != ST_TZ || g.nx % 8 != 0 || !L.vec || c.nx % 4 != 0) return false;
+    if (g.dim != 3 || g.ncell < (1LL << 21) || g.tz != ST_TZ || g.nx % 8 != 0 || !L.vec || c.nx % 4 != 0) return false;
     for (const void *p : {(const void *)L.b, (const void *)L.inv, (const void *)L.x, (const void *)L.cx,
                           (const void *)L.cy, (const void *)L.cz, (const void *)L.diag, (const void *)L.xc,
                           (const void *)S.p, (const void *)S.q})

@@ -70,9 +70,12 @@ struct Grid {
 // deep_min: the fewest cells for tiles 4 planes deep. Deep tiles give a
 // block more cells and the gather-first column kernels their 4 planes;
 // thin ones spread small grids over all SMs. A scene's fine grid takes deep
-// tiles from 2^21 cells (128^3), coarse levels only above (their 2^21-cell
-// level, under a 256^3 grid, balances better in thin tiles).
-constexpr long long DEEP_MIN_FINE = 1LL << 21;
+// tiles above 2^18 cells (64^3): mixed MGPCG with thin and deep tiles, ms, at
+// 64^3 liquid 1.66 / 1.69, 80^3 2.27 / 2.20, 96^3 2.49 / 2.39, 112^3 3.33 /
+// 3.07, a batch of 64 liquids up to 160^3 73.5 / 69.4, six served scenes 30.0 /
+// 26.9. Coarse levels take them only above 2^21 (their 2^21-cell level, under
+// a 256^3 grid, balances better in thin tiles: 11.17 against 11.25 ms).
+constexpr long long DEEP_MIN_FINE = (1LL << 18) + 1;
 constexpr long long DEEP_MIN_COARSE = (1LL << 21) + 1;
 inline Grid make_grid(int dim, int nx, int ny, int nz, long long deep_min = DEEP_MIN_FINE) {
     Grid g;
