@@ -444,9 +444,8 @@ template <class T> void Solver::add_to_plan(BatchPlan<T> &plan, const gbp_params
 template void Solver::add_to_plan<double>(BatchPlan<double> &, const gbp_params &) const;
 template void Solver::add_to_plan<float>(BatchPlan<float> &, const gbp_params &) const;
 
-int Solver::finish_batched(const gbp_params &p, cudaStream_t stream) {
+int Solver::fetch_scalars(cudaStream_t stream) {
     SOLVER_CUDA(cudaMemcpyAsync(st_.host_sc, st_.sc, sizeof(Scalars), cudaMemcpyDeviceToHost, stream));
-    SOLVER_CUDA(cudaStreamSynchronize(stream));
     return GBP_OK;
 }
 
@@ -473,7 +472,9 @@ int Solver::solve_mg(const Grid &g, const gbp_params &p, int grid_blocks, cudaSt
     }
     rc = mixed ? runner_.solve<float>(p, stream, launches) : runner_.solve<double>(p, stream, launches);
     if (rc) return fail(rc, runner_.error());
-    return finish_batched(p, stream);
+    if ((rc = fetch_scalars(stream))) return rc;
+    SOLVER_CUDA(cudaStreamSynchronize(stream));
+    return GBP_OK;
 }
 
 namespace {

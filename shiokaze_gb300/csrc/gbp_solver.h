@@ -65,8 +65,10 @@ public:
     Level0Out level0_out(const gbp_params &p) const;
     void level0_written() { level0_written_ = true; }
     template <class T> void add_to_plan(BatchPlan<T> &plan, const gbp_params &p) const;
-    // Reads this scene's scalars after a batched solve.
-    int finish_batched(const gbp_params &p, cudaStream_t stream);
+    // Enqueues a copy of this scene's scalars to host_scalars(), valid once
+    // the stream is synchronised (after a solve: what complete() reads).
+    int fetch_scalars(cudaStream_t stream);
+    const Scalars &host_scalars() const { return *st_.host_sc; }
     // After the solve: FP64 true residual, iteration counts, status
     // (GBP_OK / GBP_ERR_NOT_CONVERGED / GBP_ERR_NAN).
     int complete(const Grid &g, const gbp_params &p, int grid_blocks, cudaStream_t stream, long long *launches);
