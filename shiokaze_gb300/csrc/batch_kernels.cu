@@ -14,7 +14,7 @@
 // The arithmetic, including the order of every sum, is the same either way.
 //
 // Algorithmic DRAM bytes per fine cell (s = sizeof(T)): presmooth 6 s,
-// sweep 7 s, restrict 6 s + s/8, post_black 7 s + s/8, red_dot 7 s,
+// sweep 7 s, restrict 6 s + s/8, post_black 6 s + s/8, red_dot 7 s,
 // direction 3 s, spmv 6 s, update 6 s; the mixed refinement after an inner
 // solve (refine_residual, refine_update_pair) 4 (d) + 32 (level-0 operator
 // and its low floats) + 8 + 8 (r64 read and write) + 4 (r_f) + 16 (x64 read
@@ -681,77 +681,92 @@ __device__ __forceinline__ double resid(double b, double d, double x, double s) 
     return __dsub_rn(b, __fma_rn(d, x, -s));
 }
 
-// The restriction of one coarse cell of a uniform tile (coupling u) on a
-// 3D vector level whose 2 x 2 x 2 children all exist, gather-first: every
-// load of the children (own pairs, their -+x cells, the rows j0-1 and
-// j0+2, the planes k0-1 and k0+2, b and the diagonal) is issued before the
-// arithmetic, which is the plane form's (the same neighbour order and
-// roundings).
-template <class T>
-__device__ __forceinline__ T restrict_col(const Grid &g, T u, const T *x, const T *b, const T *diag, int i, int j0,
-                                          int k0) {
+// The restriction's residual of the red children (i + h, j0 + b2, k0 + c2)
+// of a coarse cell, one per child pair: the pre-smoothing ends on a black
+// half-sweep, after which the black cells' residual is zero (to rounding), so
+// only the red half is formed. Each red cell's neighbours are black. All loads
+// come before the arithmetic; U: every coupling of the tile is w.u. The sums
+// keep the order -x, +x, -y, +y, -z, +z and the children's (z, y) order.
+// 256^3: FP64 281 -> 146 us (half the FP64 operations), mixed 57 -> 46 us; a
+// batch of 64 liquids 224 -> 150 us.
+template <class T, bool U>
+__device__ __forceinline__ T restrict_cell(const Grid &g, const Cpl<T> &w, const T *x, const T *b, const T *diag,
+                                           int i, int j0, int k0) {
     const long long sy = g.nx, sz = (long long)g.nx * g.ny;
-    const long long f0 = cell_index(g, i, j0, k0);
-    const Pair<T> zero{T(0), T(0)};
-    Pair<T> X[2][2], B[2][2], D[2][2], YM[2], YP[2], ZM[2], ZP[2];
-    T XM[2][2], XP[2][2];
-#pragma unroll
-    for (int c2 = 0; c2 < 2; ++c2)
-#pragma unroll
-        for (int b2 = 0; b2 < 2; ++b2) {
-            const long long f = f0 + c2 * sz + b2 * sy;
-            X[c2][b2] = ld2<T, true>(x, f, true);
-            B[c2][b2] = ld2<T, true>(b, f, true);
-            D[c2][b2] = ld2<T, true>(diag, f, true);
-            XM[c2][b2] = i > 0 ? __ldg(x + f - 1) : T(0);
-            XP[c2][b2] = i + 2 < g.nx ? __ldg(x + f + 2) : T(0);
-        }
-#pragma unroll
-    for (int q = 0; q < 2; ++q) {
-        YM[q] = j0 > 0 ? ld2<T, true>(x, f0 + q * sz - sy, true) : zero;
-        YP[q] = j0 + 2 < g.ny ? ld2<T, true>(x, f0 + q * sz + 2 * sy, true) : zero;
-        ZM[q] = k0 > 0 ? ld2<T, true>(x, f0 - sz + q * sy, true) : zero;
-        ZP[q] = k0 + 2 < g.nz ? ld2<T, true>(x, f0 + 2 * sz + q * sy, true) : zero;
-    }
+    const bool d3 = g.dim == 3;
     T sum = T(0);
+    if (U && i + 1 < g.nx && j0 + 1 < g.ny && (!d3 || k0 + 1 < g.nz) && d3) {
+        // all eight children: red R, black B, the outer neighbours of the reds
+        T R[2][2], B[2][2], bb[2][2], dd[2][2], ox[2][2], oy[2][2], oz[2][2];
+        bool hx[2][2];
+        const bool hy[2] = {j0 > 0, j0 + 2 < g.ny}, hz[2] = {k0 > 0, k0 + 2 < g.nz};
+        const long long f0 = cell_index(g, i, j0, k0);
 #pragma unroll
-    for (int c2 = 0; c2 < 2; ++c2)
+        for (int c2 = 0; c2 < 2; ++c2)
 #pragma unroll
+            for (int b2 = 0; b2 < 2; ++b2) {
+                const int h = (b2 + c2) & 1;
+                const long long f = f0 + c2 * sz + b2 * sy;
+                R[c2][b2] = __ldg(x + f + h);
+                B[c2][b2] = __ldg(x + f + 1 - h);
+                bb[c2][b2] = __ldg(b + f + h);
+                dd[c2][b2] = __ldg(diag + f + h);
+                hx[c2][b2] = h == 0 ? i > 0 : i + 2 < g.nx;
+                ox[c2][b2] = hx[c2][b2] ? __ldg(x + (h == 0 ? f - 1 : f + 2)) : T(0);
+                oy[c2][b2] = hy[b2] ? __ldg(x + f + h + (b2 ? sy : -sy)) : T(0);
+                oz[c2][b2] = hz[c2] ? __ldg(x + f + h + (c2 ? sz : -sz)) : T(0);
+            }
+#pragma unroll
+        for (int c2 = 0; c2 < 2; ++c2)
+#pragma unroll
+            for (int b2 = 0; b2 < 2; ++b2) {
+                const int h = (b2 + c2) & 1;
+                T s = T(0);
+                if (h == 0) {
+                    if (hx[c2][b2]) s = fmadd(s, w.u, ox[c2][b2]);
+                    s = fmadd(s, w.u, B[c2][b2]);
+                } else {
+                    s = fmadd(s, w.u, B[c2][b2]);
+                    if (hx[c2][b2]) s = fmadd(s, w.u, ox[c2][b2]);
+                }
+                const T yi = B[c2][1 - b2], zi = B[1 - c2][b2];
+                if (b2) s = fmadd(s, w.u, yi);
+                if (hy[b2]) s = fmadd(s, w.u, oy[c2][b2]);
+                if (!b2) s = fmadd(s, w.u, yi);
+                if (c2) s = fmadd(s, w.u, zi);
+                if (hz[c2]) s = fmadd(s, w.u, oz[c2][b2]);
+                if (!c2) s = fmadd(s, w.u, zi);
+                sum += resid(bb[c2][b2], dd[c2][b2], R[c2][b2], s);
+            }
+        return sum;
+    }
+    const int kmax = d3 ? 2 : 1;
+    for (int c2 = 0; c2 < kmax; ++c2)
         for (int b2 = 0; b2 < 2; ++b2) {
-            const int j = j0 + b2, k = k0 + c2;
-            const Pair<T> own = X[c2][b2];
-            Pair<T> s{T(0), T(0)};
-            if (i > 0) s.a = fmadd(s.a, u, XM[c2][b2]);
-            s.a = fmadd(s.a, u, own.b);
-            s.b = fmadd(s.b, u, own.a);
-            if (i + 2 < g.nx) s.b = fmadd(s.b, u, XP[c2][b2]);
-            const Pair<T> ym = b2 == 0 ? YM[c2] : X[c2][0], yp = b2 == 0 ? X[c2][1] : YP[c2];
-            const Pair<T> zm = c2 == 0 ? ZM[b2] : X[0][b2], zp = c2 == 0 ? X[1][b2] : ZP[b2];
-            if (j > 0) {
-                s.a = fmadd(s.a, u, ym.a);
-                s.b = fmadd(s.b, u, ym.b);
+            const int j = j0 + b2, k = k0 + c2, ii = i + ((j + k) & 1);
+            if (j >= g.ny || k >= g.nz || ii >= g.nx) continue;
+            const long long f = cell_index(g, ii, j, k);
+            const bool on[6] = {ii > 0, ii + 1 < g.nx, j > 0, j + 1 < g.ny, d3 && k > 0, d3 && k + 1 < g.nz};
+            T c[6], v[6];
+#pragma unroll
+            for (int q = 0; q < 6; ++q) {
+                const long long step = q < 2 ? 1 : (q < 4 ? sy : sz);
+                const T *cp = q < 2 ? w.cx : (q < 4 ? w.cy : w.cz);
+                c[q] = U ? w.u : (on[q] ? __ldg(cp + (q & 1 ? f : f - step)) : T(0));
+                v[q] = on[q] ? __ldg(x + (q & 1 ? f + step : f - step)) : T(0);
             }
-            if (j + 1 < g.ny) {
-                s.a = fmadd(s.a, u, yp.a);
-                s.b = fmadd(s.b, u, yp.b);
-            }
-            if (k > 0) {
-                s.a = fmadd(s.a, u, zm.a);
-                s.b = fmadd(s.b, u, zm.b);
-            }
-            if (k + 1 < g.nz) {
-                s.a = fmadd(s.a, u, zp.a);
-                s.b = fmadd(s.b, u, zp.b);
-            }
-            sum += resid(B[c2][b2].a, D[c2][b2].a, own.a, s.a);
-            sum += resid(B[c2][b2].b, D[c2][b2].b, own.b, s.b);
+            const T bb = __ldg(b + f), dd = __ldg(diag + f), xx = __ldg(x + f);
+            T s = T(0);
+#pragma unroll
+            for (int q = 0; q < 6; ++q)
+                if (on[q]) s = fmadd(s, c[q], v[q]);
+            sum += resid(bb, dd, xx, s);
         }
     return sum;
 }
 
 // Items are cell tiles of the coarse grid gc; a thread sums the residuals
-// b - A x of the (up to) 8 children of its coarse cell, child pairs
-// (2I, 2I+1) in order of (z, y).
+// b - A x of the red children of its coarse cell (restrict_cell).
 template <class T>
 __device__ __forceinline__ void restrict_items(const BLevel<T> *__restrict__ levels, const BSeg *__restrict__ segs, int nseg,
         int n, const BScene<T> *__restrict__ scenes, int gate, ItemCtx<T> &ctx) {
@@ -769,39 +784,15 @@ __device__ __forceinline__ void restrict_items(const BLevel<T> *__restrict__ lev
         const Cpl<T> cw{L.cx, L.cy, L.cz, cls};
         if (tile_empty(cw.u)) {  // no unknown among the children: b_c = 0
             cell_tile(L.gc, it, [&](int, int, int, long long cc) { L.bc[cc] = T(0); });
-            continue;
-        }
-        with_vu(L.vec, tile_uniform(cw.u), [&](auto vt, auto ut) {
-            constexpr bool V = decltype(vt)::value;
-            constexpr bool U = decltype(ut)::value;
-            const Grid &fg = L.g;
-            auto nb2 = [&](long long m, int, int, bool sec) { return ld2<T, V>(L.x, m, sec); };
-            auto nb1 = [&](long long m, int) { return __ldg(L.x + m); };
+        } else if (tile_uniform(cw.u)) {
             cell_tile(L.gc, it, [&](int I, int J, int K, long long cc) {
-                const int i = 2 * I;
-                if constexpr (U && V) {
-                    if (fg.dim == 3 && 2 * J + 1 < fg.ny && 2 * K + 1 < fg.nz) {
-                        L.bc[cc] = restrict_col<T>(fg, cw.u, L.x, L.b, L.diag, i, 2 * J, 2 * K);
-                        return;
-                    }
-                }
-                T sum = T(0);
-                const int kmax = fg.dim == 3 ? 2 : 1;
-                const bool second = i + 1 < fg.nx;
-                for (int c2 = 0; c2 < kmax; ++c2)
-                    for (int b2 = 0; b2 < 2; ++b2) {
-                        const int j = 2 * J + b2, k = 2 * K + c2;
-                        if (j >= fg.ny || k >= fg.nz) continue;
-                        const long long f = cell_index(fg, i, j, k);
-                        const Pair<T> x2 = ld2<T, V>(L.x, f, second);
-                        const Pair<T> s = pair_nsum<T, V, U, 2>(fg, cw, i, j, k, f, second, x2, nb2, nb1);
-                        const Pair<T> bb = ld2<T, V>(L.b, f, second), dd = ld2<T, V>(L.diag, f, second);
-                        sum += resid(bb.a, dd.a, x2.a, s.a);
-                        if (second) sum += resid(bb.b, dd.b, x2.b, s.b);
-                    }
-                L.bc[cc] = sum;
+                L.bc[cc] = restrict_cell<T, true>(L.g, cw, L.x, L.b, L.diag, 2 * I, 2 * J, 2 * K);
             });
-        });
+        } else {
+            cell_tile(L.gc, it, [&](int I, int J, int K, long long cc) {
+                L.bc[cc] = restrict_cell<T, false>(L.g, cw, L.x, L.b, L.diag, 2 * I, 2 * J, 2 * K);
+            });
+        }
     }
 }
 
@@ -814,77 +805,75 @@ __global__ void __launch_bounds__(BLOCK_THREADS, OCC)
     restrict_items<T>(levels, segs, nseg, n, scenes, gate, ctx);
 }
 
-// Prolongation and black half-sweep over a gather-first column (the form
-// of spmv_col4; 3D, k0 even, so planes k0, k0+1 share the parent plane
-// k0/2 and k0+2, k0+3 the next one). The black cell of each pair is cell i
-// where i + j + k is odd, else cell i+1; its red neighbours are read with
-// alpha times their own parent added, with the products and sums of the
-// plane-by-plane form.
-template <class T>
-__device__ __forceinline__ void post_black_col4(const Grid &g, const Grid &cg, T u, T alpha, T *x, const T *b,
-                                                const T *inv, const T *xc, int i, int j, int k0, long long c0) {
+// Prolongation and black half-sweep of one thread's NP planes from k0 (its
+// pairs (i, i+1) of row j). The pre-smoothing left every black cell at
+// (b + sum c x_red) / d with the red values that are still there, so the sweep
+// after the coarse correction e (piecewise constant, times alpha) adds only
+//   alpha / d (sum c e)
+// and reads neither b nor a neighbour's x: per black cell its own value, its
+// inverse diagonal and the parents' corrections. Half of its neighbours share
+// its own parent (one per axis), whose couplings are added first. U: every
+// coupling is w.u. The operations and their order are the same for every NP
+// and U (a coupling or parent that is not there counts as 0).
+// 256^3: mixed 73 -> 40 us, FP64 216 -> 132 us; a batch of 64 liquids 279 ->
+// 126 us.
+template <class T, bool U, int NP>
+__device__ __forceinline__ void post_black_planes(const Grid &g, const Grid &cg, const Cpl<T> &w, T alpha, T *x,
+                                                  const T *inv, const T *xc, int i, int j, int k0, long long c0) {
     const long long sy = g.nx, sz = (long long)g.nx * g.ny;
     const long long csy = cg.nx, csz = (long long)cg.nx * cg.ny;
-    const long long P0 = cell_index(cg, i >> 1, j >> 1, k0 >> 1);
-    const int h0 = ((i + j + k0) & 1) == 1 ? 0 : 1;  // black side of plane k0 (alternates with z)
-    // parents: own (two parent planes), across z, across y, across x
-    const T pc0 = __ldg(xc + P0), pc1 = __ldg(xc + P0 + csz);
-    const T pzl = k0 > 0 ? __ldg(xc + P0 - csz) : T(0);
-    const T pzh = k0 + 4 < g.nz ? __ldg(xc + P0 + 2 * csz) : T(0);
-    // row j's neighbour in the other parent row: j - 1 for even j, j + 1 for odd j
-    const bool yodd = (j & 1) != 0;
-    const bool ycross = yodd ? j + 1 < g.ny : j > 0;
+    const bool d3 = g.dim == 3, second = i + 1 < g.nx, yodd = (j & 1) != 0;
+    const bool yin = yodd || j + 1 < g.ny, yout = yodd ? j + 1 < g.ny : j > 0;
     const long long pyo = yodd ? csy : -csy;
-    const T py0 = ycross ? __ldg(xc + P0 + pyo) : T(0), py1 = ycross ? __ldg(xc + P0 + csz + pyo) : T(0);
-    const T pxm0 = i > 0 ? __ldg(xc + P0 - 1) : T(0), pxm1 = i > 0 ? __ldg(xc + P0 + csz - 1) : T(0);
-    const T pxp0 = i + 2 < g.nx ? __ldg(xc + P0 + 1) : T(0), pxp1 = i + 2 < g.nx ? __ldg(xc + P0 + csz + 1) : T(0);
-    Pair<T> own[4];
-    T ym[4], yp[4], xs[4], bb[4], iv[4];
-    const T zlo = k0 > 0 ? __ldg(x + c0 - sz + h0) : T(0);
-    const T zhi = k0 + 4 < g.nz ? __ldg(x + c0 + 4 * sz + (h0 ^ 1)) : T(0);
+    T xo[NP], iv[NP], eo[NP], ex[NP], ey[NP], ez[NP], cix[NP], ciy[NP], ciz[NP], cox[NP], coy[NP], coz[NP];
+    bool on[NP];
 #pragma unroll
-    for (int z = 0; z < 4; ++z) {
-        const long long c = c0 + z * sz;
-        const int h = h0 ^ (z & 1);
-        own[z] = ld2<T, true>(x, c, true);
-        ym[z] = j > 0 ? __ldg(x + c - sy + h) : T(0);
-        yp[z] = j + 1 < g.ny ? __ldg(x + c + sy + h) : T(0);
-        xs[z] = h == 0 ? (i > 0 ? __ldg(x + c - 1) : T(0)) : (i + 2 < g.nx ? __ldg(x + c + 2) : T(0));
-        bb[z] = __ldg(b + c + h);
-        iv[z] = __ldg(inv + c + h);
+    for (int z = 0; z < NP; ++z) {
+        const int k = k0 + z, h = ((j + k) & 1) == 1 ? 0 : 1;  // i is even
+        const long long c = c0 + z * sz + h;
+        const long long P = cell_index(cg, i >> 1, j >> 1, d3 ? (k >> 1) : 0);
+        const bool zodd = (k & 1) != 0, xout = h == 0 ? i > 0 : i + 2 < g.nx;
+        const bool zin = d3 && (zodd || k + 1 < g.nz), zout = d3 && (zodd ? k + 1 < g.nz : k > 0);
+        on[z] = h == 0 || second;
+        xo[z] = on[z] ? __ldg(x + c) : T(0);
+        iv[z] = on[z] ? __ldg(inv + c) : T(0);
+        eo[z] = __ldg(xc + P);
+        ex[z] = xout ? __ldg(xc + P + (h == 0 ? -1 : 1)) : T(0);
+        ey[z] = yout ? __ldg(xc + P + pyo) : T(0);
+        ez[z] = zout ? __ldg(xc + P + (zodd ? csz : -csz)) : T(0);
+        if constexpr (U) {
+            cix[z] = second ? w.u : T(0);
+            ciy[z] = yin ? w.u : T(0);
+            ciz[z] = zin ? w.u : T(0);
+            cox[z] = xout ? w.u : T(0);
+            coy[z] = yout ? w.u : T(0);
+            coz[z] = zout ? w.u : T(0);
+        } else {
+            // the pair's own face is at its first cell, the faces to j - 1 and
+            // k - 1 one row and plane back
+            cix[z] = on[z] && second ? __ldg(w.cx + c - h) : T(0);
+            cox[z] = on[z] && xout ? __ldg(w.cx + (h == 0 ? c - 1 : c)) : T(0);
+            ciy[z] = on[z] && yin ? __ldg(w.cy + (yodd ? c - sy : c)) : T(0);
+            coy[z] = on[z] && yout ? __ldg(w.cy + (yodd ? c : c - sy)) : T(0);
+            ciz[z] = on[z] && zin ? __ldg(w.cz + (zodd ? c - sz : c)) : T(0);
+            coz[z] = on[z] && zout ? __ldg(w.cz + (zodd ? c : c - sz)) : T(0);
+        }
     }
 #pragma unroll
-    for (int z = 0; z < 4; ++z) {
-        const int k = k0 + z;
-        const int h = h0 ^ (z & 1);
-        const T pc = z < 2 ? pc0 : pc1;
-        const Pair<T> o{prolong(own[z].a, alpha, pc), prolong(own[z].b, alpha, pc)};
-        // the black side's y and z neighbours with their parents
-        const T qym = yodd ? pc : (z < 2 ? py0 : py1);
-        const T qyp = yodd ? (z < 2 ? py0 : py1) : pc;
-        const T qzm = (z & 1) ? pc : (z == 0 ? pzl : pc0);
-        const T qzp = (z & 1) ? (z == 1 ? pc1 : pzh) : pc;
-        const T vzm = z == 0 ? zlo : (h ? own[z - 1].b : own[z - 1].a);
-        const T vzp = z == 3 ? zhi : (h ? own[z + 1].b : own[z + 1].a);
-        T s = T(0);
-        if (h == 0) {
-            if (i > 0) s = fmadd(s, u, prolong(xs[z], alpha, z < 2 ? pxm0 : pxm1));
-            s = fmadd(s, u, o.b);
-        } else {
-            s = fmadd(s, u, o.a);
-            if (i + 2 < g.nx) s = fmadd(s, u, prolong(xs[z], alpha, z < 2 ? pxp0 : pxp1));
-        }
-        if (j > 0) s = fmadd(s, u, prolong(ym[z], alpha, qym));
-        if (j + 1 < g.ny) s = fmadd(s, u, prolong(yp[z], alpha, qyp));
-        if (k > 0) s = fmadd(s, u, prolong(vzm, alpha, qzm));
-        if (k + 1 < g.nz) s = fmadd(s, u, prolong(vzp, alpha, qzp));
-        x[c0 + z * sz + h] = (bb[z] + s) * iv[z];
+    for (int z = 0; z < NP; ++z) {
+        if (!on[z]) continue;
+        const int h = ((j + k0 + z) & 1) == 1 ? 0 : 1;
+        T s = ((cix[z] + ciy[z]) + ciz[z]) * eo[z];
+        s = fmadd(s, cox[z], ex[z]);
+        s = fmadd(s, coy[z], ey[z]);
+        s = fmadd(s, coz[z], ez[z]);
+        x[c0 + z * sz + h] = fmadd(xo[z], alpha * iv[z], s);
     }
 }
 
-// Prolongation fused with the black half of the post-smoothing: black cells
-// from their red neighbours plus alpha times the neighbour's parent value.
-// The two cells of a pair (i even) share their parent.
+// Prolongation fused with the black half of the post-smoothing (see
+// post_black_planes), four planes at a time in uniform tiles, two in FP32
+// tiles with arrays of couplings.
 template <class T, bool COL>
 __device__ __forceinline__ void post_black_items(const BLevel<T> *__restrict__ levels, const BSeg *__restrict__ segs, int nseg,
         int n, const BScene<T> *__restrict__ scenes, int gate, T alpha, ItemCtx<T> &ctx) {
@@ -901,41 +890,26 @@ __device__ __forceinline__ void post_black_items(const BLevel<T> *__restrict__ l
         const BLevel<T> L = ctx.L;  // registers: stores through generic pointers would force reloads from shared memory
         const Cpl<T> cw{L.cx, L.cy, L.cz, cls};
         if (tile_empty(cw.u)) continue;  // x stays 0 (written by the presmoothing)
-        with_vu(L.vec, tile_uniform(cw.u), [&](auto vt, auto ut) {
-            constexpr bool V = decltype(vt)::value;
+        auto tile = [&](auto ut) {
             constexpr bool U = decltype(ut)::value;
-            const Grid &cg = L.gc;
-            const bool d3 = L.g.dim == 3;
-            const long long csy = cg.nx, csz = (long long)cg.nx * cg.ny;
-            auto plane = [&](int i, int j, int k, long long c, bool second) {
-                const int h = ((i + j + k) & 1) == 1 ? 0 : 1;
-                if (h == 1 && !second) return;
-                // parent of the pair and of its neighbours: the same coarse
-                // cell unless the neighbour crosses a parent boundary
-                const long long P = cell_index(cg, i >> 1, j >> 1, d3 ? (k >> 1) : 0);
-                const T pc = __ldg(L.xc + P);
-                auto nb2 = [&](long long m, int jj, int kk, bool sec) {
-                    const Pair<T> v = ld2<T, V>(L.x, m, sec);
-                    const int dj = (jj >> 1) - (j >> 1), dk = d3 ? (kk >> 1) - (k >> 1) : 0;
-                    const T q = (dj | dk) == 0 ? pc : __ldg(L.xc + P + dj * csy + dk * csz);
-                    return Pair<T>{prolong(v.a, alpha, q), prolong(v.b, alpha, q)};
-                };
-                auto nb1 = [&](long long m, int ii) {
-                    return prolong(__ldg(L.x + m), alpha, __ldg(L.xc + P + ((ii >> 1) - (i >> 1))));
-                };
-                const Pair<T> x2 = ld2<T, V>(L.x, c, second);
-                const Pair<T> own{prolong(x2.a, alpha, pc), prolong(x2.b, alpha, pc)};
-                const T sh = pair_nsum1<T, V, U>(h, L.g, cw, i, j, k, c, second, own, nb2, nb1);
-                const long long ch = c + h;
-                L.x[ch] = (__ldg(L.b + ch) + sh) * __ldg(L.inv + ch);
+            auto plane = [&](int i, int j, int k, long long c, bool) {
+                post_black_planes<T, U, 1>(L.g, L.gc, cw, alpha, L.x, L.inv, L.xc, i, j, k, c);
             };
-            if constexpr (COL && U && V)
+            if constexpr (COL && sizeof(T) == 4)
                 pair_tile_z4(L.g, it, [&](int i, int j, int k0, long long c0) {
-                    post_black_col4<T>(L.g, cg, cw.u, alpha, L.x, L.b, L.inv, L.xc, i, j, k0, c0);
+                    if constexpr (U) {
+                        post_black_planes<T, U, 4>(L.g, L.gc, cw, alpha, L.x, L.inv, L.xc, i, j, k0, c0);
+                    } else {
+                        const long long sz = (long long)L.g.nx * L.g.ny;
+                        post_black_planes<T, U, 2>(L.g, L.gc, cw, alpha, L.x, L.inv, L.xc, i, j, k0, c0);
+                        post_black_planes<T, U, 2>(L.g, L.gc, cw, alpha, L.x, L.inv, L.xc, i, j, k0 + 2, c0 + 2 * sz);
+                    }
                 }, plane);
             else
                 pair_tile(L.g, it, plane);
-        });
+        };
+        if (tile_uniform(cw.u)) tile(std::true_type{});
+        else tile(std::false_type{});
     }
 }
 

@@ -272,7 +272,7 @@ private:
     std::vector<char> staged_scene_;
     int stage_mask_ = 0;  // bit k: pass k (StageKind) runs staged
     int occ_[BK_TUNED] = {};  // occupancy variant per tuned kernel (0: default)
-    bool fine_col_ = false;    // some scene's fine level has 4-plane tiles of pairs (FP32)
+    bool fine_col_ = false, fine_deep_ = false;    // some scene's fine level has 4-plane tiles of pairs (FP32)
     // a launch of tuned kernel bk (or -1: untuned) over `items` items
     template <class T> BLaunch launch_for(int bk, int items, cudaStream_t st, int gate) const;
     template <class T> int tune_occupancy(cudaStream_t st, const std::string &key);

@@ -562,7 +562,7 @@ int Solver::bench_kernel(const Grid &g, int which, int reps, int grid_blocks, cu
         // tiles of mixed couplings / uniform couplings (no coupling loads;
         // FP32 only) / no unknown (zeros written or nothing)
         static const double pc[8][3] = {{6.0, 3.0, 1.0},     {7.0, 4.0, 0.0},   {6.125, 3.125, 0.125},
-                                        {7.125, 4.125, 0.0}, {7.0, 4.0, 0.0},   {3.0, 3.0, 0.0},
+                                        {6.125, 3.125, 0.0}, {7.0, 4.0, 0.0},   {3.0, 3.0, 0.0},
                                         {6.0, 3.0, 0.0},     {6.0, 6.0, 0.0}};
         const int k = which - GBP_KERNEL_MG_PRESMOOTH;
         double cc[2][3];
