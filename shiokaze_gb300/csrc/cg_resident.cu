@@ -23,8 +23,8 @@
 // the solve is done again by the launched form.
 //
 // Measured on one GB300 (launched form, one launch with FP64 trees, this):
-// 2D liquid 128^2, 575 iterations, 9.37 / 5.64 / 4.08 ms; 3D liquid
-// 75 x 92 x 61, 1057 iterations, 47.9 / 21.1 / 13.2 ms.
+// 2D liquid 128^2, 575 iterations, 9.37 / 5.64 / TP ms; 3D liquid
+// 75 x 92 x 61, 1057 iterations, 47.9 / 21.1 / TR ms.
 //
 // Waits: the cluster form uses the hardware barrier; the cooperative form
 // polls, bounded, and leaves with status 4 if a wait runs out.
