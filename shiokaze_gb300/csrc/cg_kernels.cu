@@ -16,6 +16,7 @@
 //   spmv    read s (8) + diag,cx,cy,cz (32), write z (8)            = 48 B
 //   update  read x,s,r,z (32), write x,r (16)                       = 48 B
 //   dir     read r,s (16), write s (8)                              = 24 B
+#include "cg_persistent.cuh"
 #include "gbp_internal.cuh"
 #include "gbp_kernels.h"
 
@@ -266,6 +267,24 @@ cudaError_t launch_cg_iteration(const Grid &g, Operator<double> A, double *x, do
     cg_update_kernel<<<nb, BLOCK_THREADS, 0, stream>>>(g, x, r, s, z, sc, pt);
     cg_direction_kernel<<<nb, BLOCK_THREADS, 0, stream>>>(g, r, s, sc);
     return cudaGetLastError();
+}
+
+bool cg_persistent_fits(const Grid &g, int grid_blocks) {
+    const int nb = blocks_for(g, grid_blocks);
+    const long long per = (g.ntiles + nb - 1) / nb * g.tz;
+    return g.ncell < (1LL << 31) && per <= 64 && cg_persistent_plan(nb, (int)per, grid_blocks / 6).use;
+}
+
+cudaError_t launch_cg_persistent(const Grid &g, Operator<double> A, double *x, double *r, double *s, Scalars *sc,
+                                 Partials *pt, int grid_blocks, cudaStream_t stream) {
+    const int nb = blocks_for(g, grid_blocks);
+    CgPersistentPlan p = cg_persistent_plan(nb, (int)((g.ntiles + nb - 1) / nb * g.tz), grid_blocks / 6);
+    p.args.x = x;
+    p.args.r = r;
+    p.args.s = s;
+    p.args.sc = sc;
+    p.args.pt = pt;
+    return cg_persistent_launch(p, cgp::GridRows{g, A}, stream);
 }
 
 cudaError_t launch_cg_spmv(const Grid &g, Operator<double> A, const double *s, double *z, Scalars *sc, Partials *pt,

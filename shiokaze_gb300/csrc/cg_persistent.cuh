@@ -27,6 +27,7 @@
 #pragma once
 
 #include "gbp_internal.cuh"
+#include "gbp_kernels.h"
 
 namespace gbp {
 
@@ -45,6 +46,48 @@ struct CgPersistentArgs {
 namespace cgp {
 
 constexpr int kPolls = 1 << 22;  // about two seconds
+// Rows of the matrix-free operator: thread t of virtual block vb has the
+// cells of tiles vb, vb + nb, ..., tz planes each, as for_each_cell walks them.
+struct GridRows {
+    Grid g;
+    Operator<double> A;
+    // the cell of item c and its neighbours that exist (bits 0..5: -x +x -y +y -z +z); -1: none, or not an unknown
+    __device__ __forceinline__ int row(int vb, int nb, int c, int t, unsigned &nbr) const {
+        const int q = g.tz == 1 ? c : c / g.tz;
+        const long long tile = vb + (long long)q * nb;
+        if (tile >= g.ntiles) return -1;
+        int i, j, k;
+        tile_origin(g, tile, i, j, k);
+        i += t & (TILE_X - 1);
+        j += t / TILE_X;
+        k += c - q * g.tz;
+        if (i >= g.nx || j >= g.ny || k >= g.nz) return -1;
+        const int e = (int)cell_index(g, i, j, k);
+        nbr = (i > 0 ? 1u : 0u) | (i + 1 < g.nx ? 2u : 0u) | (j > 0 ? 4u : 0u) | (j + 1 < g.ny ? 8u : 0u) |
+              (g.dim == 3 && k > 0 ? 16u : 0u) | (g.dim == 3 && k + 1 < g.nz ? 32u : 0u);
+        // a cell off the unknowns has a zero row, r, s and x
+        return (__double_as_longlong(__ldg(A.diag + e)) << 1) != 0 ? e : -1;
+    }
+    // apply_A's terms in its order, every load first
+    __device__ __forceinline__ double apply(int e, unsigned nbr, double s, const double *sv) const {
+        const int sy = g.nx, sz = g.nx * g.ny;
+        double c[6], v[6];
+#pragma unroll
+        for (int n = 0; n < 6; ++n) {
+            const int step = n < 2 ? 1 : (n < 4 ? sy : sz);
+            const double *cp = n < 2 ? A.cx : (n < 4 ? A.cy : A.cz);
+            const bool on = nbr >> n & 1u;
+            c[n] = on ? __ldg(cp + (n & 1 ? e : e - step)) : 0.0;
+            v[n] = on ? __ldcg(sv + (n & 1 ? e + step : e - step)) : 0.0;
+        }
+        double acc = __ldg(A.diag + e) * s;
+#pragma unroll
+        for (int n = 0; n < 6; ++n)
+            if (nbr >> n & 1u) acc = fma(-c[n], v[n], acc);
+        return acc;
+    }
+};
+
 // Rows of a matrix in compressed rows, as for_each_row walks them
 struct CsrRows {
     long long n;
@@ -301,7 +344,7 @@ inline CgPersistentPlan cg_persistent_plan(int nb, int per_block, int sms) {
     p.args.rounds = (each + p.args.sub - 1) / p.args.sub;
     p.args.nb = nb;
     p.args.per_block = per_block;
-    p.args.max_steps = 4096;
+    p.args.max_steps = CG_PERSISTENT_STEPS;
     p.threads = p.args.sub * BLOCK_THREADS;
     const size_t items = (size_t)p.args.rounds * per_block * p.threads;
     p.shared = items * (4 * sizeof(double) + 2 * sizeof(int)) +

@@ -238,7 +238,7 @@ cudaError_t csr_cg_run(CsrWork &w, long long n, double residual, int max_iter, i
         plan.args.s = w.s;
         plan.args.sc = w.sc;
         plan.args.pt = w.pt;
-        for (int left = max_iter; e == cudaSuccess; left -= plan.args.max_steps) {
+        for (int left = max_iter; e == cudaSuccess; left -= CG_PERSISTENT_STEPS) {
             if ((e = cg_persistent_launch(plan, cgp::CsrRows{n, w.rowstart, w.cols, w.vals}, stream)) != cudaSuccess)
                 break;
             *launches += 1;

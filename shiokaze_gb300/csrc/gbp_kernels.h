@@ -86,16 +86,14 @@ cudaError_t launch_cg_init(const Grid &g, Operator<double> A, const double *b, c
 // beta; s = r + beta s. Three launches; all return at once after the stop.
 cudaError_t launch_cg_iteration(const Grid &g, Operator<double> A, double *x, double *r, double *s, double *z,
                                 Scalars *sc, Partials *pt, int grid_blocks, cudaStream_t stream);
-// The whole solve in one launch (cg_resident.cu), after launch_cg_init:
-// whether a grid is tried, and one launch of it, which ends with sc->done or
-// after CG_RESIDENT_STEPS iterations. `list` is one int a cell of scratch.
-// Status 4: a wait between blocks ran out; 5 and 6: the solve has to be done
-// by the launched form from launch_cg_init on (a sum left the range its
-// fixed-point form holds; the unknowns do not fit the shared memory).
-constexpr int CG_RESIDENT_STEPS = 4096;
-bool cg_resident_grid(const Grid &g);
-cudaError_t launch_cg_resident(const Grid &g, Operator<double> A, double *x, double *r, double *s, void *list,
-                               Scalars *sc, Partials *pt, int grid_blocks, cudaStream_t stream);
+// The whole solve in one launch (cg_persistent.cuh), the same bits as the
+// iterations: whether a grid's vectors fit, and one launch of it, which ends
+// with sc->done or after a few thousand iterations (status 4: a wait between
+// blocks ran out).
+constexpr int CG_PERSISTENT_STEPS = 4096;  // iterations in one launch
+bool cg_persistent_fits(const Grid &g, int grid_blocks);
+cudaError_t launch_cg_persistent(const Grid &g, Operator<double> A, double *x, double *r, double *s, Scalars *sc,
+                                 Partials *pt, int grid_blocks, cudaStream_t stream);
 // The three launches of an iteration, one at a time (benchmarking).
 cudaError_t launch_cg_spmv(const Grid &g, Operator<double> A, const double *s, double *z, Scalars *sc, Partials *pt,
                            int grid_blocks, cudaStream_t stream);

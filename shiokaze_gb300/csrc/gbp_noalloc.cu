@@ -117,38 +117,17 @@ extern "C" int gbp_project_device_static(int dim, int nx, int ny, int nz, double
         NOALLOC_CUDA(launch_surface_tension(g, dt, dx, sp, p.surface_tension, fluid, u, v, w, grid_blocks, st));
     NOALLOC_CUDA(launch_assemble(g, dt, dx, sp, solid, fluid, u, v, w, diag, cx, cy, cz, b, sc, grid_blocks, st));
     Operator<double> A{diag, cx, cy, dim == 3 ? cz : cy};
-    // the same solve as gbp_project_device's: one launch where it takes the
-    // grid, else (or where it gives up) the launched iterations
     NOALLOC_CUDA(launch_cg_init(g, A, b, nullptr, x, r, s, sc, pt, p.residual, p.max_iterations, grid_blocks, st));
+    const int chunk = p.iterations_per_sync > 0 ? p.iterations_per_sync : 16;
     Scalars h;
     std::memset(&h, 0, sizeof(h));
-    bool launched_form = !cg_resident_grid(g);
-    for (int left = p.max_iterations; !launched_form; left -= CG_RESIDENT_STEPS) {
-        const cudaError_t e = launch_cg_resident(g, A, x, r, s, z, sc, pt, grid_blocks, st);
-        if (e == cudaErrorCooperativeLaunchTooLarge) {
-            cudaGetLastError();
-            launched_form = true;
-            break;
-        }
-        NOALLOC_CUDA(e);
+    const long long max_chunks = (long long)p.max_iterations / chunk + 2;
+    for (long long k = 0; k < max_chunks; ++k) {
         NOALLOC_CUDA(cudaMemcpyAsync(&h, sc, sizeof(Scalars), cudaMemcpyDeviceToHost, st));
         NOALLOC_CUDA(cudaStreamSynchronize(st));
-        if (h.status == 4) return fail(GBP_ERR_CUDA, "gbp_project_device_static: a wait between blocks ran out");
-        if (h.status > 4) launched_form = true;
-        if (h.done || left <= 0) break;
-    }
-    if (launched_form) {
-        if (cg_resident_grid(g))
-            NOALLOC_CUDA(launch_cg_init(g, A, b, nullptr, x, r, s, sc, pt, p.residual, p.max_iterations, grid_blocks, st));
-        const int chunk = p.iterations_per_sync > 0 ? p.iterations_per_sync : 16;
-        const long long max_chunks = (long long)p.max_iterations / chunk + 2;
-        for (long long k = 0; k < max_chunks; ++k) {
-            NOALLOC_CUDA(cudaMemcpyAsync(&h, sc, sizeof(Scalars), cudaMemcpyDeviceToHost, st));
-            NOALLOC_CUDA(cudaStreamSynchronize(st));
-            if (h.done) break;
-            for (int it = 0; it < chunk; ++it)
-                NOALLOC_CUDA(launch_cg_iteration(g, A, x, r, s, z, sc, pt, grid_blocks, st));
-        }
+        if (h.done) break;
+        for (int it = 0; it < chunk; ++it)
+            NOALLOC_CUDA(launch_cg_iteration(g, A, x, r, s, z, sc, pt, grid_blocks, st));
     }
     NOALLOC_CUDA(launch_true_residual(g, A, b, x, nullptr, sc, pt, grid_blocks, st));
     NOALLOC_CUDA(launch_pressure(g, diag, x, nullptr, pressure, nullptr, grid_blocks, st));

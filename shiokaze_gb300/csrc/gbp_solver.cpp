@@ -281,28 +281,23 @@ int Solver::complete(const Grid &g, const gbp_params &p, int grid_blocks, cudaSt
 int Solver::solve_cg(const Grid &g, const gbp_params &p, int grid_blocks, cudaStream_t stream, long long *launches) {
     const bool warm = p.warm_start && st_.have_prev;
     Operator<double> A{st_.diag, st_.cx, st_.cy, g.dim == 3 ? st_.cz : st_.cy};
-    auto init = [&]() {
-        *launches += 1;
-        return launch_cg_init(g, A, st_.b, warm ? st_.prev : nullptr, st_.x, st_.r, st_.s, st_.sc, st_.pt, p.residual,
-                              p.max_iterations, grid_blocks, stream);
-    };
-    SOLVER_CUDA(init());
-    if (cg_resident_grid(g)) {
+    SOLVER_CUDA(launch_cg_init(g, A, st_.b, warm ? st_.prev : nullptr, st_.x, st_.r, st_.s, st_.sc, st_.pt,
+                               p.residual, p.max_iterations, grid_blocks, stream));
+    *launches += 1;
+    if (cg_persistent_fits(g, grid_blocks)) {
         cudaError_t e = cudaSuccess;
-        for (int left = p.max_iterations;; left -= CG_RESIDENT_STEPS) {
-            e = launch_cg_resident(g, A, st_.x, st_.r, st_.s, st_.z, st_.sc, st_.pt, grid_blocks, stream);
-            // blocks that cannot be resident together (a partitioned GPU): the launched form
-            if (e == cudaErrorCooperativeLaunchTooLarge) break;
-            SOLVER_CUDA(e);
+        for (int left = p.max_iterations; e == cudaSuccess; left -= CG_PERSISTENT_STEPS) {
+            e = launch_cg_persistent(g, A, st_.x, st_.r, st_.s, st_.sc, st_.pt, grid_blocks, stream);
+            if (e != cudaSuccess) break;
             *launches += 1;
             SOLVER_CUDA(cudaMemcpyAsync(st_.host_sc, st_.sc, sizeof(Scalars), cudaMemcpyDeviceToHost, stream));
             SOLVER_CUDA(cudaStreamSynchronize(stream));
             if (st_.host_sc->status == 4) return fail(GBP_ERR_CUDA, "CG: a wait between the blocks of the solve ran out");
-            if (st_.host_sc->status > 4) break;
             if (st_.host_sc->done || left <= 0) return GBP_OK;
         }
-        if (e != cudaSuccess) cudaGetLastError();
-        SOLVER_CUDA(init());
+        // blocks that cannot be resident together (a partitioned GPU): the launched form
+        if (e != cudaErrorCooperativeLaunchTooLarge) SOLVER_CUDA(e);
+        cudaGetLastError();
     }
     const int chunk = p.iterations_per_sync > 0 ? p.iterations_per_sync : 16;
     const long long key = ((long long)chunk << 20) | ((long long)grid_blocks << 4) | 0;
