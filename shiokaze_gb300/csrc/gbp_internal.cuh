@@ -77,6 +77,7 @@ struct Grid {
 // a 256^3 grid, balances better in thin tiles: 11.17 against 11.25 ms).
 constexpr long long DEEP_MIN_FINE = (1LL << 18) + 1;
 constexpr long long DEEP_MIN_COARSE = (1LL << 21) + 1;
+constexpr long long DEEP_MIN_CG = 1LL << 21;  // plain CG (Solver::solve_cg)
 inline Grid make_grid(int dim, int nx, int ny, int nz, long long deep_min = DEEP_MIN_FINE) {
     Grid g;
     g.dim = dim;

@@ -100,7 +100,7 @@ extern "C" int gbp_project_device_static(int dim, int nx, int ny, int nz, double
     if (rc) return rc;
     cudaStream_t st = (cudaStream_t)stream;
 
-    const Grid g = make_grid(dim, nx, ny, nz);
+    const Grid g = make_grid(dim, nx, ny, nz, DEEP_MIN_CG);
     double *vec[9];
     for (int i = 0; i < 9; ++i) vec[i] = reinterpret_cast<double *>(base + (size_t)i * kVecBytes);
     double *diag = vec[0], *cx = vec[1], *cy = vec[2], *cz = vec[3], *b = vec[4];

@@ -278,7 +278,11 @@ int Solver::complete(const Grid &g, const gbp_params &p, int grid_blocks, cudaSt
     return GBP_OK;
 }
 
-int Solver::solve_cg(const Grid &g, const gbp_params &p, int grid_blocks, cudaStream_t stream, long long *launches) {
+int Solver::solve_cg(const Grid &grid, const gbp_params &p, int grid_blocks, cudaStream_t stream, long long *launches) {
+    // CG's tiles stay one plane deep below 2^21 cells: they give its sums their
+    // order, which decides (through CG's growth of rounding differences) where
+    // a solve stops
+    const Grid g = make_grid(grid.dim, grid.nx, grid.ny, grid.nz, DEEP_MIN_CG);
     const bool warm = p.warm_start && st_.have_prev;
     Operator<double> A{st_.diag, st_.cx, st_.cy, g.dim == 3 ? st_.cz : st_.cy};
     SOLVER_CUDA(launch_cg_init(g, A, st_.b, warm ? st_.prev : nullptr, st_.x, st_.r, st_.s, st_.sc, st_.pt,
