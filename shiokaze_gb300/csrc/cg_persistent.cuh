@@ -2,28 +2,39 @@
 // systems whose vectors fit the SMs' shared memory.
 //
 // The launched form of CG (cg_kernels.cu, csr_solver.cu) takes three launches
-// an iteration, whose time on a small system is latency: the launch, the
-// partial sums read back by the last block, and a shuffle tree in every warp
-// on the FP64 pipe (a warp instruction holds it 16 cycles). Here the blocks
-// stay resident, keep x, r, s and z of their rows in shared memory, exchange
-// s through L2 and meet at three barriers an iteration. Measured on one
-// GB300, launched and here: 2D liquid 128^2 (one cluster) 9.37 and 5.64 ms for
-// 575 iterations, 3D liquid 75 x 92 x 61 47.9 and 21.1 ms for 1057, a 64^3
-// liquid's matrix in rows 21.5 and 12.3 ms for 920. What bounds it now is the
-// latency of dependent FP64 operations (over 100 cycles a level of the sums'
-// trees, 800 for a division) and the L2 round trips of the barriers.
+// an iteration, whose time on a small system is latency. Here the blocks stay
+// resident, keep x, r, s and z of their rows in shared memory and exchange s
+// through L2.
 //
-// Results equal the launched form's bit for bit: the rows, the order in which
-// a thread adds them, and the shape of every sum are the same. The work is
-// cut into the launched form's blocks of 256 threads ("virtual blocks"); a
-// physical block carries `sub` of them side by side, `rounds` times over, and
-// every virtual block sums its 256 values in block_sum's tree, the partials
-// in reduce_partials_sum's. Virtual blocks without a row keep partial 0.
-// The maximum is order-free; it runs on integers (bit patterns of the
-// absolute values), off the FP64 pipe.
+// Results equal the launched form's bit for bit, as they have to: CG from
+// these right-hand sides multiplies a difference of 1e-15 to 3e-4 in thirty
+// iterations, so a sum in another order stops elsewhere. The rows, the order
+// in which a thread adds its terms and the shape of every sum are therefore
+// the launched form's: the work is cut into its blocks of 256 threads
+// ("virtual blocks"); a physical block carries `sub` of them, and every virtual
+// block sums its 256 values in block_sum's tree, the partials in
+// reduce_partials_sum's. Virtual blocks without a row keep partial 0. What
+// need not keep that shape does not: the stencil and the vector updates run
+// over the block's rows packed into full warps (of the 32 x 8 tiles of a
+// liquid many lanes have none), and the stop test is a flag, the sign bit of
+// the partial of r.r.
+//
+// Exchange of the partials: a cluster's blocks push them into each other's
+// shared memory and meet at the hardware barrier; blocks of a cooperative
+// launch write them to L2, meet at a counter and read them all. (Polling the
+// slots themselves instead of the counter, 379 to 912 of them from 152 blocks,
+// held up the writes: 17.8 against 12.3 ms on the matrix below.)
+//
+// Measured on one GB300, launched form and here: 2D liquid 128^2 (a cluster)
+// 9.37 and 5.2 ms for 575 iterations, 3D liquid 75 x 92 x 61 47.9 and 21.0 ms
+// for 1057, a 64^3 liquid's matrix in rows 21.5 and 12.0 ms for 920. (One
+// thread a lane of the virtual blocks instead of packed rows, partials through
+// L2 in the cluster too: 5.6, 21.1 and 12.3 ms.) What is left is latency: over
+// 100 cycles a level of the FP64 trees, 800 for each of the two divisions, and
+// the L2 round trips.
 //
 // Waits: the cluster form uses the hardware barrier; the cooperative form
-// polls a counter, bounded, and leaves with status 4 if a wait runs out.
+// polls, bounded, and leaves with status 4 if a wait runs out.
 #pragma once
 
 #include "gbp_internal.cuh"
@@ -34,10 +45,9 @@ namespace gbp {
 struct CgPersistentArgs {
     double *x, *r, *s;
     Scalars *sc;
-    Partials *pt;
+    Partials *pt;   // the partials of s.z (a) and r.r (c)
     int nb;         // virtual blocks, as many as the launched form has blocks
-    int sub;        // virtual blocks side by side in a physical block
-    int rounds;     // virtual blocks one after the other
+    int sub;        // virtual blocks of a physical block
     int per_block;  // rows a thread has in one virtual block (the launched form's tiles and planes)
     int max_steps;  // iterations in this launch
 };
@@ -46,6 +56,8 @@ struct CgPersistentArgs {
 namespace cgp {
 
 constexpr int kPolls = 1 << 22;  // about two seconds
+constexpr int kClusterBlocks = 16, kClusterSlots = 64;
+
 // Rows of the matrix-free operator: thread t of virtual block vb has the
 // cells of tiles vb, vb + nb, ..., tz planes each, as for_each_cell walks them.
 struct GridRows {
@@ -106,11 +118,10 @@ struct CsrRows {
             const int m = (int)(e1 - q < 8 ? e1 - q : 8);
             double a[8], v[8];
 #pragma unroll
-            for (int n = 0; n < 8; ++n)
-                if (n < m) {
-                    a[n] = __ldg(vals + q + n);
-                    v[n] = __ldcg(sv + __ldg(cols + q + n));
-                }
+            for (int n = 0; n < 8; ++n) {
+                a[n] = n < m ? __ldg(vals + q + n) : 0.0;
+                v[n] = n < m ? __ldcg(sv + __ldg(cols + q + n)) : 0.0;
+            }
 #pragma unroll
             for (int n = 0; n < 8; ++n)
                 if (n < m) acc = fma(a[n], v[n], acc);
@@ -144,174 +155,201 @@ template <bool CLUSTER> __device__ __forceinline__ bool meet(unsigned *count, un
 }
 
 template <class Rows, bool CLUSTER>
-__global__ void __launch_bounds__(CLUSTER ? 1024 : 768, 1) cg_persistent_kernel(const Rows rows, const CgPersistentArgs a) {
+__global__ void __launch_bounds__(CLUSTER ? 512 : 768, 1) cg_persistent_kernel(const Rows rows, const CgPersistentArgs a) {
     extern __shared__ double smem[];
     Scalars *sc = a.sc;
     if (sc->done) return;
-    const int T = blockDim.x, tid = threadIdx.x, items = a.rounds * a.per_block;
-    double *R = smem + tid, *S = R + items * T, *Z = S + items * T, *X = Z + items * T;
-    double *red = smem + 4 * items * T;                    // padded values of every virtual block
-    double *fin = red + a.rounds * a.sub * TREE_PAD;           // the partials' 256 strided sums
-    int *meta = (int *)(fin + TREE_PAD) + tid;                 // row and neighbour bits of each item
-    unsigned *nbrs = (unsigned *)((int *)(fin + TREE_PAD) + items * T) + tid;
-    __shared__ unsigned long long smax[32];
-    __shared__ int active[32];  // virtual blocks with rows: r * sub + s
-    __shared__ int has[32];
-    __shared__ double sh_alpha, sh_beta;
-    __shared__ int sh_done, n_active;
-    const int sub = tid >> 8, t = tid & 255, warp = tid >> 5, lane = tid & 31, nwarps = T >> 5;
-    auto virtual_block = [&](int r, int s) { return (int)blockIdx.x + (int)gridDim.x * (s + a.sub * r); };
+    const int T = blockDim.x, tid = threadIdx.x, nvb = a.sub, slots = nvb * a.per_block * 256;
+    // home order: virtual block, item, thread
+    double *R = smem, *S = R + slots, *Z = S + slots, *X = Z + slots;
+    double *red = smem + 4 * slots;                // padded values of every virtual block
+    double *fin = red + nvb * TREE_PAD;            // the partials' 256 strided sums
+    double *box = fin + TREE_PAD;                  // the cluster's partials, by parity
+    int *cell = (int *)(box + 2 * kClusterSlots);  // the block's rows packed: row,
+    int *home = cell + slots;                      // slot << 6 | neighbour bits
+    __shared__ int warp_n[32], active[32], has[32];
+    __shared__ double sh_scalar;
+    __shared__ int sh_status, sh_large, n_active, n_rows;
+    const int warp = tid >> 5, lane = tid & 31, nwarps = T >> 5;
+    auto virtual_block = [&](int q) { return (int)blockIdx.x + (int)gridDim.x * q; };
     if (tid < 32) has[tid] = 0;
+    if (tid == 0) n_rows = 0, sh_large = 0;
     __syncthreads();
-    for (int r = 0; r < a.rounds; ++r) {
-        const int vb = virtual_block(r, sub);
-        bool any = false;
-        for (int c = 0; c < a.per_block; ++c) {
-            const int m = (r * a.per_block + c) * T;
-            unsigned nbr = 0;
-            const int e = vb < a.nb ? rows.row(vb, a.nb, c, t, nbr) : -1;
-            meta[m] = e;
-            nbrs[m] = nbr;
-            if (e >= 0) {
-                any = true;
-                R[m] = a.r[e];
-                S[m] = a.s[e];
-                X[m] = a.x[e];
-            }
+    // the block's rows, packed in home order
+    for (int h0 = 0; h0 < slots; h0 += T) {
+        const int h = h0 + tid;
+        int e = -1, q = 0;
+        unsigned nbr = 0;
+        if (h < slots) {
+            q = h / (a.per_block * 256);
+            const int rest = h - q * a.per_block * 256, vb = virtual_block(q);
+            if (vb < a.nb) e = rows.row(vb, a.nb, rest >> 8, rest & 255, nbr);
+            R[h] = e >= 0 ? a.r[e] : 0.0;
+            S[h] = e >= 0 ? a.s[e] : 0.0;
+            X[h] = e >= 0 ? a.x[e] : 0.0;
+            Z[h] = 0.0;
+            if (e >= 0) has[q] = 1;
         }
-        if (any) has[r * a.sub + sub] = 1;
+        const unsigned vote = __ballot_sync(0xffffffffu, e >= 0);
+        if (lane == 0) warp_n[warp] = __popc(vote);
+        __syncthreads();
+        const int mine = lane < nwarps ? warp_n[lane] : 0;
+        const int at = n_rows + __reduce_add_sync(0xffffffffu, lane < warp ? mine : 0) + __popc(vote & ((1u << lane) - 1u));
+        if (e >= 0) {
+            cell[at] = e;
+            home[at] = h << 6 | (int)nbr;
+        }
+        const int all = __reduce_add_sync(0xffffffffu, mine);
+        __syncthreads();
+        if (tid == 0) n_rows += all;
+        __syncthreads();
     }
-    __syncthreads();
     if (tid == 0) {
         int n = 0;
-        for (int q = 0; q < a.rounds * a.sub; ++q) {
-            const int vb = virtual_block(q / a.sub, q % a.sub);
-            if (has[q]) {
-                active[n++] = q;
-            } else if (vb < a.nb) {
-                a.pt->a[vb] = 0.0;
-                a.pt->c[vb] = 0.0;
-            }
-        }
+        for (int q = 0; q < nvb; ++q)
+            if (has[q]) active[n++] = q;
         n_active = n;
     }
-    double rho = sc->rho, res = sc->res, alpha = 0.0, beta = sc->beta;
-    const double tol = sc->tol;
-    int iter = sc->iter, status = 0;
+    // virtual blocks without a row have partial 0
+    if (CLUSTER) {
+        for (int q = tid; q < 2 * kClusterSlots; q += T) box[q] = 0.0;
+    } else if (tid < nvb && !has[tid] && virtual_block(tid) < a.nb) {
+        __stcg(a.pt->a + virtual_block(tid), 0.0);
+        __stcg(a.pt->c + virtual_block(tid), 0.0);
+    }
+    double rho = sc->rho, alpha = 0.0, beta = sc->beta;
+    const unsigned long long tol = abs_bits(sc->tol);
+    int iter = sc->iter, status = 0, sums = 0;
     const int max_iter = sc->max_iter;
     unsigned target = 0;
     unsigned *count = &sc->counter[4];
-    __syncthreads();
-    bool good = true;
+    bool good = meet<CLUSTER>(count, target);
 
-    // one partial per virtual block with rows, by a warp each
-    auto partials = [&](double *out) {
+    // Every thread's items of the active virtual blocks, term by term in
+    // order, then the trees: a partial per virtual block (negative if `large`)
+    // to every block.
+    auto partials = [&](auto term, bool large, double *out) {
+        if (large) sh_large = 1;
         __syncthreads();
-        for (int q = warp; q < n_active; q += nwarps) {
-            const double s = tree256(red + active[q] * TREE_PAD);
-            if (lane == 0) __stcg(out + virtual_block(active[q] / a.sub, active[q] % a.sub), s);
+        for (int v = tid; v < n_active * 256; v += T) {
+            const int q = active[v >> 8], t = v & 255;
+            double sum = 0.0;
+            for (int c = 0; c < a.per_block; ++c) sum = term((q * a.per_block + c) * 256 + t, sum);
+            red[q * TREE_PAD + tree_at(t)] = sum;
+        }
+        __syncthreads();
+        const bool mark = sh_large != 0;
+        for (int n = warp; n < n_active; n += nwarps) {
+            const int q = active[n], vb = virtual_block(q);
+            double p = tree256(red + q * TREE_PAD);
+            if (mark) p = -p;
+            if (CLUSTER) {
+                p = __shfl_sync(0xffffffffu, p, 0);
+                if (lane < (int)gridDim.x) {
+                    const unsigned mine = (unsigned)__cvta_generic_to_shared(box + (sums & 1) * kClusterSlots + vb);
+                    unsigned to;
+                    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(to) : "r"(mine), "r"(lane));
+                    asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(to), "d"(p) : "memory");
+                }
+            } else if (lane == 0) {
+                __stcg(out + vb, p);
+            }
         }
     };
-    // reduce_partials_sum, in every block alike; valid in thread 0
-    auto total = [&](const double *p) {
+    // reduce_partials_sum, in every block alike: valid in thread 0. With
+    // `marks` the partials are magnitudes and any tells whether one came
+    // marked. False if a wait ran out.
+    auto total = [&](double &sum, bool &any, const double *in, bool marks) {
+        if (!meet<CLUSTER>(count, target)) return false;
+        if (tid == 0) sh_large = 0;
+        int marked = 0;
         if (tid < 256) {
             double v = 0.0;
-            for (int q = tid; q < a.nb; q += 256) v += __ldcg(p + q);
+            for (int q = tid; q < a.nb; q += 256) {
+                double p = CLUSTER ? box[(sums & 1) * kClusterSlots + q] : __ldcg(in + q);
+                if (marks) {
+                    marked |= __double_as_longlong(p) < 0;
+                    p = fabs(p);
+                }
+                v += p;
+            }
             fin[tree_at(tid)] = v;
         }
-        __syncthreads();
-        return warp == 0 ? tree256(fin) : 0.0;
+        ++sums;
+        any = __syncthreads_or(marked) != 0;
+        sum = warp == 0 ? tree256(fin) : 0.0;
+        return true;
     };
 
-    for (int step = 0; step < a.max_steps; ++step) {
+    double r2 = sc->r2;
+    for (int step = 0; good && step < a.max_steps; ++step) {
         // z = A s, s.z
-        for (int r = 0; r < a.rounds; ++r) {
-            double dot = 0.0;
-            for (int c = 0; c < a.per_block; ++c) {
-                const int m = (r * a.per_block + c) * T;
-                if (meta[m] < 0) continue;
-                const double z = rows.apply(meta[m], nbrs[m], S[m], a.s);
-                Z[m] = z;
-                dot = fma(S[m], z, dot);
-            }
-            if (has[r * a.sub + sub]) red[(r * a.sub + sub) * TREE_PAD + tree_at(t)] = dot;
+        for (int e = tid; e < n_rows; e += T) {
+            const int h = home[e] >> 6;
+            Z[h] = rows.apply(cell[e], (unsigned)home[e] & 63u, S[h], a.s);
         }
-        partials(a.pt->a);
-        if (!(good = meet<CLUSTER>(count, target))) break;
-        const double pap = total(a.pt->a);
-        if (tid == 0) sh_alpha = rho / pap;
+        bool more;
+        double pap, rho_new;
+        partials([&](int h, double sum) { return fma(S[h], Z[h], sum); }, false, a.pt->a);
+        good = total(pap, more, a.pt->a, false);
+        if (!good) break;
+        if (tid == 0) sh_scalar = rho / pap;
         __syncthreads();
-        alpha = sh_alpha;
-        // x += alpha s, r -= alpha z, |r|_inf, r.r
-        unsigned long long mx = 0;
-        for (int r = 0; r < a.rounds; ++r) {
-            double r2 = 0.0;
-            for (int c = 0; c < a.per_block; ++c) {
-                const int m = (r * a.per_block + c) * T;
-                if (meta[m] < 0) continue;
-                X[m] = fma(alpha, S[m], X[m]);
-                const double rv = fma(-alpha, Z[m], R[m]);
-                R[m] = rv;
-                const unsigned long long b = abs_bits(rv);
-                mx = b > mx ? b : mx;
-                r2 = fma(rv, rv, r2);
-            }
-            if (has[r * a.sub + sub]) red[(r * a.sub + sub) * TREE_PAD + tree_at(t)] = r2;
+        alpha = sh_scalar;
+        // x += alpha s, r -= alpha z, r.r, whether |r| exceeds the threshold
+        bool large = false;
+        for (int e = tid; e < n_rows; e += T) {
+            const int h = home[e] >> 6;
+            X[h] = fma(alpha, S[h], X[h]);
+            const double rv = fma(-alpha, Z[h], R[h]);
+            R[h] = rv;
+            large = large || abs_bits(rv) > tol;
         }
-        mx = warp_max_bits(mx);
-        if (lane == 0) smax[warp] = mx;
-        partials(a.pt->c);
-        if (warp == nwarps - 1) {
-            mx = warp_max_bits(lane < nwarps ? smax[lane] : 0ull);
-            if (lane == 0) __stcg((unsigned long long *)a.pt->b + blockIdx.x, mx);
-        }
-        if (!(good = meet<CLUSTER>(count, target))) break;
-        unsigned long long gm = 0;
-        if (warp == 0) {
-            for (int q = lane; q < (int)gridDim.x; q += 32) {
-                const unsigned long long b = __ldcg((const unsigned long long *)a.pt->b + q);
-                gm = b > gm ? b : gm;
-            }
-            gm = warp_max_bits(gm);
-        }
-        const double rho_new = total(a.pt->c);
+        partials([&](int h, double sum) { return fma(R[h], R[h], sum); }, large, a.pt->c);
+        good = total(rho_new, more, a.pt->c, true);
+        if (!good) break;
         ++iter;
         if (tid == 0) {
-            res = __longlong_as_double((long long)gm);
-            int done = 0;
-            if (res <= tol) done = 1;
-            else if (iter >= max_iter) done = 2;
-            else if (rho_new != rho_new || alpha != alpha) done = 3;
-            sh_beta = rho_new / rho;
-            sc->r2 = rho_new;  // every block writes the same value
-            if (!done) rho = rho_new;
-            sh_done = done;
+            r2 = rho_new;
+            sh_status = !more ? 1 : (iter >= max_iter ? 2 : (rho_new != rho_new || alpha != alpha ? 3 : 0));
+            sh_scalar = rho_new / rho;
+            if (!sh_status) rho = rho_new;
         }
         __syncthreads();
-        status = sh_done;
+        status = sh_status;
         if (status) break;
-        beta = sh_beta;
+        beta = sh_scalar;
         // s = r + beta s
-        for (int m = 0; m < items * T; m += T) {
-            if (meta[m] < 0) continue;
-            const double s = fma(beta, S[m], R[m]);
-            S[m] = s;
-            __stcg(a.s + meta[m], s);
+        for (int e = tid; e < n_rows; e += T) {
+            const int h = home[e] >> 6;
+            const double s = fma(beta, S[h], R[h]);
+            S[h] = s;
+            __stcg(a.s + cell[e], s);
         }
-        if (step + 1 < a.max_steps && !(good = meet<CLUSTER>(count, target))) break;
-    }
-    for (int m = 0; m < items * T; m += T) {
-        if (meta[m] < 0) continue;
-        a.x[meta[m]] = X[m];
-        a.r[meta[m]] = R[m];
+        good = meet<CLUSTER>(count, target);
     }
     if (!good) status = 4;
-    if ((blockIdx.x == 0 || !good) && tid == 0) {
-        sc->rho = rho;
-        sc->alpha = alpha;
-        sc->beta = beta;
-        sc->res = res;
-        sc->iter = iter;
+    if (status < 4) {
+        unsigned long long mx = 0;
+        for (int e = tid; e < n_rows; e += T) {
+            const int h = home[e] >> 6;
+            a.x[cell[e]] = X[h];
+            a.r[cell[e]] = R[h];
+            mx = max(mx, abs_bits(R[h]));
+        }
+        mx = warp_max_bits(mx);
+        if (lane == 0 && mx) atomicMax(&sc->bits_max, mx);
+        if (!meet<CLUSTER>(count, target)) status = 4;
+    }
+    if ((blockIdx.x == 0 || status == 4) && tid == 0) {
+        if (status < 4) {
+            sc->rho = rho;
+            sc->r2 = r2;
+            sc->alpha = alpha;
+            sc->beta = beta;
+            sc->res = __longlong_as_double((long long)__ldcg(&sc->bits_max));
+            sc->iter = iter;
+        }
         sc->status = status;
         sc->done = status != 0;
     }
@@ -322,10 +360,9 @@ __global__ void __launch_bounds__(CLUSTER ? 1024 : 768, 1) cg_persistent_kernel(
 
 // Shape of a persistent solve of nb virtual blocks with per_block rows a
 // thread: up to 64 virtual blocks (the 2D grids, 24^3) run as one cluster of
-// 16 blocks of at most four, whose hardware barrier beats a polled counter;
-// larger ones as a cooperative grid of one block an SM, three virtual blocks
-// side by side (85 registers a thread). Used while x, r, s, z and the row
-// table fit the shared memory (about 900,000 grid cells); beyond, the launched
+// 16 blocks, whose barrier and shared memory beat L2; larger ones as
+// a cooperative grid of one block an SM. Used while x, r, s, z and the row
+// table fit the shared memory (about 800,000 grid cells); beyond, the launched
 // form's passes are long enough to hide their launches.
 struct CgPersistentPlan {
     bool use = false, cluster = false;
@@ -338,18 +375,15 @@ inline CgPersistentPlan cg_persistent_plan(int nb, int per_block, int sms) {
     CgPersistentPlan p;
     p.cluster = nb <= 64;
     p.blocks = p.cluster ? 16 : (nb < sms ? nb : sms);
-    while (p.cluster && p.blocks > 1 && p.blocks / 2 >= nb) p.blocks /= 2;
     const int each = (nb + p.blocks - 1) / p.blocks;
-    p.args.sub = each < (p.cluster ? 4 : 3) ? each : (p.cluster ? 4 : 3);
-    p.args.rounds = (each + p.args.sub - 1) / p.args.sub;
+    p.args.sub = each;
     p.args.nb = nb;
     p.args.per_block = per_block;
     p.args.max_steps = CG_PERSISTENT_STEPS;
-    p.threads = p.args.sub * BLOCK_THREADS;
-    const size_t items = (size_t)p.args.rounds * per_block * p.threads;
-    p.shared = items * (4 * sizeof(double) + 2 * sizeof(int)) +
-               ((size_t)p.args.rounds * p.args.sub + 1) * TREE_PAD * sizeof(double);
-    p.use = p.shared <= 220 * 1024 && p.args.rounds * p.args.sub <= 32 && nb <= MAX_GRID;
+    p.threads = p.cluster ? 512 : 768;
+    const size_t slots = (size_t)each * per_block * 256;
+    p.shared = slots * (4 * sizeof(double) + 2 * sizeof(int)) + (((size_t)each + 1) * TREE_PAD + 2 * 64) * sizeof(double);
+    p.use = p.shared <= 216 * 1024 && each <= 32 && nb <= MAX_GRID;
     return p;
 }
 
@@ -361,6 +395,8 @@ cudaError_t cg_persistent_launch(const CgPersistentPlan &p, const Rows &rows, cu
                                : (const void *)cgp::cg_persistent_kernel<Rows, false>;
     cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.shared);
     if (e == cudaSuccess && p.cluster) e = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    // the maximum, and the barrier's count
+    if (e == cudaSuccess) e = cudaMemsetAsync(&p.args.sc->bits_max, 0, sizeof(unsigned long long), stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(&p.args.sc->counter[4], 0, sizeof(unsigned), stream);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg{};
@@ -369,20 +405,18 @@ cudaError_t cg_persistent_launch(const CgPersistentPlan &p, const Rows &rows, cu
     cfg.dynamicSmemBytes = p.shared;
     cfg.stream = stream;
     cudaLaunchAttribute at[1];
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
     if (p.cluster) {
         at[0].id = cudaLaunchAttributeClusterDimension;
         at[0].val.clusterDim.x = (unsigned)p.blocks;
         at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
         int n = 0;
-        cfg.attrs = at;
-        cfg.numAttrs = 1;
         if ((e = cudaOccupancyMaxActiveClusters(&n, fn, &cfg)) != cudaSuccess) return e;
         if (n < 1) return cudaErrorCooperativeLaunchTooLarge;
     } else {
         at[0].id = cudaLaunchAttributeCooperative;
         at[0].val.cooperative = 1;
-        cfg.attrs = at;
-        cfg.numAttrs = 1;
     }
     Rows r = rows;
     CgPersistentArgs a = p.args;
