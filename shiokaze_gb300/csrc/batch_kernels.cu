@@ -15,7 +15,8 @@
 //
 // Algorithmic DRAM bytes per fine cell (s = sizeof(T)): presmooth 6 s,
 // sweep 7 s, restrict 6 s + s/8, post_black 6 s + s/8, red_dot 7 s,
-// direction 3 s, spmv 6 s, update 6 s; the mixed refinement after an inner
+// direction and product 9 s in one pass (staged levels: direction 3 s, spmv
+// 6 s), update 6 s; the mixed refinement after an inner
 // solve (refine_residual, refine_update_pair) 4 (d) + 32 (level-0 operator
 // and its low floats) + 8 + 8 (r64 read and write) + 4 (r_f) + 16 (x64 read
 // and write) = 72 B.
@@ -1078,6 +1079,63 @@ __device__ __forceinline__ void spmv_col4(const Grid &g, T u, const T *p, const 
     }
 }
 
+// p = z + beta p, q = A z + beta q and p . q over a column (direction_spmv):
+// A z is r on the red cells, the stencil's sum of red neighbours on the black
+template <class T>
+__device__ __forceinline__ void direction_spmv_col4(const Grid &g, T u, const T *zv, const T *rv, const T *diag, T *pv,
+                                                    T *qv, T beta, bool fresh, int i, int j, int k0, long long c0,
+                                                    DotAcc<T> &acc) {
+    const long long sy = g.nx, sz = (long long)g.nx * g.ny;
+    const Pair<T> zero{T(0), T(0)};
+    Pair<T> own[4], po[4], qo[4];
+    T xs[4], ym[4], yp[4], rr[4], dv[4];
+    const int h0 = (i + j + k0 + 1) & 1;  // black side of plane k0 (alternates with z)
+    const T zlo = k0 > 0 ? __ldg(zv + c0 - sz + h0) : T(0);
+    const T zhi = k0 + 4 < g.nz ? __ldg(zv + c0 + 4 * sz + (h0 ^ 1)) : T(0);
+#pragma unroll
+    for (int z = 0; z < 4; ++z) {
+        const long long c = c0 + z * sz;
+        const int hb = h0 ^ (z & 1);
+        own[z] = ld2<T, true>(zv, c, true);
+        ym[z] = j > 0 ? __ldg(zv + c - sy + hb) : T(0);
+        yp[z] = j + 1 < g.ny ? __ldg(zv + c + sy + hb) : T(0);
+        xs[z] = hb == 0 ? (i > 0 ? __ldg(zv + c - 1) : T(0)) : (i + 2 < g.nx ? __ldg(zv + c + 2) : T(0));
+        rr[z] = __ldg(rv + c + (hb ^ 1));
+        dv[z] = __ldg(diag + c + hb);
+        po[z] = fresh ? zero : ld2<T, true>(pv, c, true);
+        qo[z] = fresh ? zero : ld2<T, true>(qv, c, true);
+    }
+#pragma unroll
+    for (int z = 0; z < 4; ++z) {
+        const int k = k0 + z;
+        const int hb = h0 ^ (z & 1);
+        const T zm = z == 0 ? zlo : (hb ? own[z - 1].b : own[z - 1].a);
+        const T zp = z == 3 ? zhi : (hb ? own[z + 1].b : own[z + 1].a);
+        T s = T(0);
+        if (hb == 0) {
+            if (i > 0) s = fmadd(s, u, xs[z]);
+            s = fmadd(s, u, own[z].b);
+        } else {
+            s = fmadd(s, u, own[z].a);
+            if (i + 2 < g.nx) s = fmadd(s, u, xs[z]);
+        }
+        if (j > 0) s = fmadd(s, u, ym[z]);
+        if (j + 1 < g.ny) s = fmadd(s, u, yp[z]);
+        if (k > 0) s = fmadd(s, u, zm);
+        if (k + 1 < g.nz) s = fmadd(s, u, zp);
+        const T az = fmadd(-s, dv[z], hb ? own[z].b : own[z].a);
+        Pair<T> p2 = own[z], q2{hb ? rr[z] : az, hb ? az : rr[z]};
+        if (!fresh) {
+            p2 = Pair<T>{fmadd(p2.a, beta, po[z].a), fmadd(p2.b, beta, po[z].b)};
+            q2 = Pair<T>{fmadd(q2.a, beta, qo[z].a), fmadd(q2.b, beta, qo[z].b)};
+        }
+        st2<T, true>(pv, c0 + z * sz, p2, true);
+        st2<T, true>(qv, c0 + z * sz, q2, true);
+        acc.add(p2.a, q2.a);
+        acc.add(p2.b, q2.b);
+    }
+}
+
 // red half-sweep of x (b = r) and z . r over a column (red_dot): the red
 // cell of each pair is cell i where i + j + k is even, else cell i+1; its
 // neighbours are black and not written here
@@ -1605,6 +1663,84 @@ __global__ void __launch_bounds__(BLOCK_THREADS, OCC)
                 if constexpr (COL && U && V)
                     pair_tile_z4(L.g, it, [&](int i, int j, int k0, long long c0) {
                         spmv_col4<T>(L.g, cw.u, S.p, L.diag, S.q, i, j, k0, c0, acc);
+                    }, plane);
+                else
+                    pair_tile(L.g, it, plane);
+            });
+        },
+        [&](const BItem &it, int flushes) {
+            Scalars *sc = ctx.S.sc;
+            if (item_last(&sc->counter[SITE_SPMV], flushes)) {
+                const double pq = sum_range(part, it.begin, flushes, shf);
+                if (threadIdx.x == 0) {
+                    sc->pap = pq;
+                    sc->alpha = sc->rho / pq;
+                    sc->counter[SITE_SPMV] = 0;
+                }
+            }
+        });
+}
+
+// The new direction and its product in one pass: p = z + beta p and, by the
+// same recurrence, q = A p = A z + beta q (beta = 0: p = z, q = A z). The
+// V-cycle ends on a red half-sweep, which solves the red rows of A z = r, so
+// A z is r there and the stencil runs on the black cells only. Two passes
+// (p, then the stencil of p: the staged fine levels still take them) move 6
+// words a cell (+ 3 couplings in mixed tiles) and take 9 FP64 operations; this
+// one 6 (+ 3) and 6.5, in one launch. The FP64 solver is bound by its
+// operations: a 256^3 solve went from 19.8 to 19.2 ms; the small ones by
+// launches and latency: 32^3 mixed 1.03 to 0.98 ms, six served scenes 22.2 to
+// 21.8 ms. At 256^3 mixed and in the batch of 64, bound by instructions, the
+// two forms take the same time.
+template <class T, int OCC, bool COL>
+__global__ void __launch_bounds__(BLOCK_THREADS, OCC)
+    direction_spmv_kernel(const BLevel<T> *__restrict__ levels, const BSeg *__restrict__ segs, int nseg, int n,
+                          const BScene<T> *__restrict__ scenes, int gate, double *part, const BatchCounters *live) {
+    if (batch_idle(live)) return;
+    __shared__ double shf[BLOCK_THREADS / 32];
+    __shared__ ItemCtx<T> ctx;
+    reduce_items<T, DotAcc<T>>(
+        segs, nseg, n, part, levels, scenes, gate, ctx,
+        [&](const BItem &it, DotAcc<T> &acc, T cls) {
+            const BLevel<T> L = ctx.L;  // registers: stores through generic pointers would force reloads from shared memory
+            const BScene<T> S = ctx.S;
+            const Cpl<T> cw{L.cx, L.cy, L.cz, cls};
+            // no unknown: p and q are read nowhere (z = 0 there)
+            if (tile_empty(cw.u)) return;
+            const T beta = T(ctx.beta);
+            const bool fresh = beta == T(0);
+            with_vu(L.vec, tile_uniform(cw.u), [&](auto vt, auto ut) {
+                constexpr bool V = decltype(vt)::value;
+                constexpr bool U = decltype(ut)::value;
+                auto nb2 = [&](long long m, int, int, bool sec) { return ld2<T, V>(S.z, m, sec); };
+                auto nb1 = [&](long long m, int) { return __ldg(S.z + m); };
+                auto plane = [&](int i, int j, int k, long long c, bool second) {
+                    const int hb = ((i + j + k) & 1) ^ 1;  // black side
+                    Pair<T> p2 = ld2<T, V>(S.z, c, second), po{T(0), T(0)}, qo{T(0), T(0)};
+                    if (!fresh) {
+                        po = ld2<T, V>(S.p, c, second);
+                        qo = ld2<T, V>(S.q, c, second);
+                    }
+                    const T rr = hb == 1 || second ? __ldg(S.r + c + (hb ^ 1)) : T(0);
+                    T az = T(0);
+                    if (hb == 0 || second) {
+                        const T d = __ldg(L.diag + c + hb);
+                        const T s = pair_nsum1<T, V, U>(hb, L.g, cw, i, j, k, c, second, p2, nb2, nb1);
+                        az = fmadd(-s, d, hb ? p2.b : p2.a);
+                    }
+                    Pair<T> q2{hb ? rr : az, hb ? az : rr};
+                    if (!fresh) {
+                        p2 = Pair<T>{fmadd(p2.a, beta, po.a), fmadd(p2.b, beta, po.b)};
+                        q2 = Pair<T>{fmadd(q2.a, beta, qo.a), fmadd(q2.b, beta, qo.b)};
+                    }
+                    st2<T, V>(S.p, c, p2, second);
+                    st2<T, V>(S.q, c, q2, second);
+                    acc.add(p2.a, q2.a);
+                    if (second) acc.add(p2.b, q2.b);
+                };
+                if constexpr (COL && U && V)
+                    pair_tile_z4(L.g, it, [&](int i, int j, int k0, long long c0) {
+                        direction_spmv_col4<T>(L.g, cw.u, S.z, S.r, L.diag, S.p, S.q, beta, fresh, i, j, k0, c0, acc);
                     }, plane);
                 else
                     pair_tile(L.g, it, plane);
@@ -2508,6 +2644,12 @@ cudaError_t b_spmv(const BLaunch &L, const BLevel<T> *levels, const BSeg *segs, 
     return cudaGetLastError();
 }
 template <class T>
+cudaError_t b_direction_spmv(const BLaunch &L, const BLevel<T> *levels, const BSeg *segs, int nseg, int n,
+                             const BScene<T> *scenes, double *part) {
+    OCC_COL_DISPATCH(L, direction_spmv_kernel, T, (levels, segs, nseg, n, scenes, L.gate, part, L.cnt));
+    return cudaGetLastError();
+}
+template <class T>
 cudaError_t b_update(const BLaunch &L, const BLevel<T> *levels, const BSeg *segs, int nseg, int n,
                      const BScene<T> *scenes, double *part, int mode, BatchCounters *cnt) {
     OCC_DISPATCH(L, update_kernel, T, (levels, segs, nseg, n, scenes, L.gate, part, mode, cnt,
@@ -2545,6 +2687,8 @@ cudaError_t b_refine_residual(const BLaunch &L, const BLevel<T> *levels, const B
                                         const BScene<T> *);                                                          \
     template cudaError_t b_spmv<T>(const BLaunch &, const BLevel<T> *, const BSeg *, int, int, const BScene<T> *,   \
                                    double *);                                                                        \
+    template cudaError_t b_direction_spmv<T>(const BLaunch &, const BLevel<T> *, const BSeg *, int, int,            \
+                                             const BScene<T> *, double *);                                           \
     template cudaError_t b_update<T>(const BLaunch &, const BLevel<T> *, const BSeg *, int, int, const BScene<T> *, \
                                      double *, int, BatchCounters *);                                                \
     template cudaError_t b_refine_residual<T>(const BLaunch &, const BLevel<T> *, const BSeg *, int, int,           \

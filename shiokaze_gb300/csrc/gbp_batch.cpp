@@ -361,6 +361,7 @@ template <class T> int BatchRunner::tune_occupancy(cudaStream_t st, const std::s
     constexpr int kVariants = 3, kRounds = 5;
     const int variants[kVariants] = {4, 5, 6};
     for (int k = 0; k < BK_TUNED && err == cudaSuccess; ++k) {
+        if (k == BK_DIRECTION && one_pass_direction()) continue;
         float t[kVariants][kRounds] = {};
         for (int v = 0; v < kVariants && err == cudaSuccess; ++v) {
             occ_[k] = variants[v];
@@ -481,7 +482,10 @@ template <class T> cudaError_t BatchRunner::fine_pass(int kind, const gbp_params
     case STAGE_PRESMOOTH: return b_presmooth<T>(L, lv, segs, nseg, n, sc);
     case STAGE_POST_BLACK: return b_post_black<T>(L, lv, segs, nseg, n, sc, T(ms.alpha));
     case STAGE_RED_DOT: return b_red_dot<T>(L, lv, segs, nseg, n, sc, d_part_);
-    default: return b_spmv<T>(L, lv, segs, nseg, n, sc, d_part_);
+    default:
+        // (the staged levels' product reads p, which its own pass formed)
+        return one_pass_direction() ? b_direction_spmv<T>(L, lv, segs, nseg, n, sc, d_part_)
+                                    : b_spmv<T>(L, lv, segs, nseg, n, sc, d_part_);
     }
 }
 
@@ -535,13 +539,15 @@ template <class T> cudaError_t BatchRunner::enqueue_iteration(const gbp_params &
         ++*nodes;
     }
     // CG on the fine level
-    if (e == cudaSuccess)
+    if (e == cudaSuccess && !one_pass_direction()) {
         e = b_direction<T>(launch_for<T>(BK_DIRECTION, n_fine_pairs_, st, gate), lv, d_fine_pairs_, s_fine_pairs_,
                            n_fine_pairs_, sc);
+        ++*nodes;
+    }
     if (e == cudaSuccess) e = fine_pass<T>(STAGE_SPMV, p, st, gate);
     if (e == cudaSuccess)
         e = b_update<T>(L(n_fine_pairs_), lv, d_fine_pairs_, s_fine_pairs_, n_fine_pairs_, sc, d_part_, mixed_ ? 1 : 0, d_counters_);
-    *nodes += 3;
+    *nodes += 2;
     if (mixed_ && e == cudaSuccess) {
         const BLaunch L2{blocks_for(n_fine_pairs_, grid_blocks_), st, 2, d_scene_of_, d_counters_};
         // x64 += d, r64 -= A d and the outer stopping rule, in one pass

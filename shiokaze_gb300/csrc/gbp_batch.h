@@ -218,7 +218,8 @@ public:
     template <class T> int solve(const gbp_params &p, cudaStream_t stream, long long *launches);
     // Times reps launches of one kernel of the iteration (benchmarking):
     // 0 presmooth, 1 restrict, 2 post_black, 3 red_dot (fine level),
-    // 4 direction, 5 spmv, 6 update.
+    // 4 direction (a pass of its own only where levels run staged), 5 spmv
+    // (with the direction in the same pass otherwise), 6 update.
     template <class T> int bench(int which, int reps, cudaStream_t stream, float *ms);
     void release();
     const char *error() const { return err_.c_str(); }
@@ -228,6 +229,8 @@ public:
         return stage_mask_ && s >= 0 && s < (int)staged_scene_.size() && staged_scene_[s];
     }
     int stage_mask() const { return stage_mask_; }
+    // the direction and its product run as one pass (no staged level)
+    bool one_pass_direction() const { return n_fine_staged_ == 0; }
     // Test hook for the next solve only (see BatchCounters::test_what):
     // makes one block's bounded waits run out, polling at most `polls`.
     void set_wait_test(int what, int block, int polls) {
@@ -333,6 +336,9 @@ cudaError_t b_direction(const BLaunch &L, const BLevel<T> *levels, const BSeg *s
 template <class T>
 cudaError_t b_spmv(const BLaunch &L, const BLevel<T> *levels, const BSeg *segs, int nseg, int n, const BScene<T> *scenes,
                    double *part);
+template <class T>
+cudaError_t b_direction_spmv(const BLaunch &L, const BLevel<T> *levels, const BSeg *segs, int nseg, int n,
+                             const BScene<T> *scenes, double *part);
 template <class T>
 cudaError_t b_update(const BLaunch &L, const BLevel<T> *levels, const BSeg *segs, int nseg, int n, const BScene<T> *scenes,
                      double *part, int mode, BatchCounters *cnt);

@@ -8,9 +8,9 @@
 //
 //   CG     (reference solver)  init; [spmv, update, direction] x chunk
 //   MGPCG  FP64                init (r = b - A prev); [V-cycle + dot,
-//                              direction, spmv, update] x chunk
-//   MGPCG  mixed               FP64 init; [FP32 V-cycle + dot, direction,
-//                              spmv, update (inner stop), x64 += d,
+//                              direction with spmv, update] x chunk
+//   MGPCG  mixed               FP64 init; [FP32 V-cycle + dot, direction
+//                              with spmv, update (inner stop), x64 += d,
 //                              r64 = b - A64 x64 (outer stop)] x chunk
 #include "gbp_solver.h"
 
@@ -572,8 +572,12 @@ int Solver::bench_kernel(const Grid &g, int which, int reps, int grid_blocks, cu
         double cc[2][3];
         if (mixed) class_cells(h32_, cc);
         else class_cells(h64_, cc);
+        // direction and product in one pass: z, p, q in, half of r and of the
+        // diagonal, the black cells' couplings; p, q out
+        static const double one_pass[3] = {9.0, 6.0, 0.0};
+        const double *words = which == GBP_KERNEL_PCG_SPMV && runner_.one_pass_direction() ? one_pass : pc[k];
         const int a = which == GBP_KERNEL_MG_RESTRICT ? 1 : 0;
-        *bytes = s * (pc[k][0] * cc[a][0] + pc[k][1] * cc[a][1] + pc[k][2] * cc[a][2]);
+        *bytes = s * (words[0] * cc[a][0] + words[1] * cc[a][1] + words[2] * cc[a][2]);
         const int rk = map[k];
         int rc = mixed ? runner_.bench<float>(rk, reps, stream, ms) : runner_.bench<double>(rk, reps, stream, ms);
         if (rc) return fail(rc, runner_.error());

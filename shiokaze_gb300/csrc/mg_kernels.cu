@@ -32,8 +32,10 @@
 //                    written); counted as a full pass                 7 s
 //   restrict         read x, b, diag, cx, cy, cz; write b_c / 8      6 s + s/8
 //   post_black       read x, x_c / 8, b, inv, cx, cy, cz; write half x  7 s
-//   direction        read z, p; write p                               3 s
-//   spmv             read p, diag, cx, cy, cz; write q                6 s
+//   direction, spmv  read z, p, q, half of r and of diag, cx, cy, cz;
+//                    write p, q                                       9 s
+//                    (staged levels, two passes: read z, p; write p, 3 s,
+//                    then read p, diag, cx, cy, cz; write q, 6 s)
 //   update           read x, p, r, q; write x, r                      6 s
 #include <algorithm>
 
