@@ -189,4 +189,85 @@ __host__ __device__ __forceinline__ bool mul_round(const MulConst c, float f, fl
     return true;
 }
 
+// A double constant as a pair of floats (within 2^-48 of it) for quot_round;
+// hi = 0 where the pair's products could leave the normal floats.
+struct PairConst {
+    float hi, lo;
+};
+inline PairConst make_pair_const(double a) {
+    const double m = a < 0 ? -a : a;
+    if (!(m >= 9.1e-13 && m <= 1.0e12)) return PairConst{0.0f, 0.0f};
+    const float hi = (float)a;
+    return PairConst{hi, (float)(a - (double)hi)};
+}
+__host__ __device__ __forceinline__ float ex_fmaf(float a, float b, float c) {
+#ifdef __CUDA_ARCH__
+    return __fmaf_rn(a, b, c);
+#else
+    return __builtin_fmaf(a, b, c);
+#endif
+}
+__host__ __device__ __forceinline__ float ex_divf(float a, float b) {
+#ifdef __CUDA_ARCH__
+    return __fdiv_rn(a, b);
+#else
+    return a / b;
+#endif
+}
+
+// The float nearest a f / rho for a constant a (dt / dx), where the FP64
+// evaluation of it (a few roundings of 2^-53) must round alike: the float pair
+// v + t is within 2^-45 of the real value (f hi exactly by an FMA, 2^-48 each
+// for lo, the sums and the quotient's correction), and the test moves it by
+// 2^-43 either way. False if the two differ (about 2^-19 of all f; up to half
+// of them where a is nearly a fraction like 3/4, whose products are ties) or a
+// value leaves the ranges; the caller then evaluates in FP64. No contraction is
+// meant here: the sources that include this are built without it.
+__host__ __device__ __forceinline__ bool quot_round(const PairConst c, float f, float rho, float &out) {
+    float v = f * c.hi;
+    if (f == 0.0f && c.hi != 0.0f) {  // a signed zero
+        out = v;
+        return true;
+    }
+    float t = ex_fmaf(f, c.lo, ex_fmaf(f, c.hi, -v));
+    float m = ex_float(ex_bits(v) & 0x7fffffffu);
+    if (!(m >= 8.7e-19f && m <= 1.1e18f)) return false;
+    if (rho != 1.0f) {
+        if (!(rho >= 9.0e-13f && rho <= 1.0f)) return false;
+        const float q = ex_divf(v, rho);
+        t = ex_divf(ex_fmaf(-q, rho, v) + t, rho);
+        v = q;
+        m = ex_float(ex_bits(v) & 0x7fffffffu);
+    }
+    const float w = m * 1.1368684e-13f;  // 2^-43
+    const float lo = v + (t - w), hi = v + (t + w);
+    out = hi;
+    return lo == hi;
+}
+
+// 1/d as a pair of doubles, r the nearest double to 1/d, for div_round.
+struct RecipConst {
+    double d, r, rlo;
+};
+// The double nearest x / d: a quotient q0 within less than one unit in the
+// last place (the reciprocal pair), its exact remainder, and one correction by
+// the nearest double to 1/d, which by Markstein's theorem (Computation of
+// elementary functions on the IBM RISC System/6000, IBM J. Res. Dev. 34, 1990)
+// rounds the quotient correctly. Four operations of the FP64 pipe where a
+// division takes several times that. For finite x with |x| 0 or in
+// [2^-300, 2^300] and d in [2^-500, 2^500]; a quotient of -0 may come as +0.
+__host__ __device__ __forceinline__ double div_round(const RecipConst c, double x) {
+#ifdef __CUDA_ARCH__
+    const double q0 = __fma_rn(x, c.r, __dmul_rn(x, c.rlo));
+    return __fma_rn(__fma_rn(-q0, c.d, x), c.r, q0);
+#else
+    const double q0 = __builtin_fma(x, c.r, x * c.rlo);
+    return __builtin_fma(__builtin_fma(-q0, c.d, x), c.r, q0);
+#endif
+}
+inline RecipConst make_recip_const(double d) {
+    const double r = 1.0 / d;
+    return RecipConst{d, r, __builtin_fma(-r, d, 1.0) * r};
+}
+
 }  // namespace gbp

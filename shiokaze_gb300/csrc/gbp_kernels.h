@@ -26,7 +26,8 @@ struct FaceArrays {
     // written only where the cell pass cannot form them from rho, area and
     // the face velocity: the weight dt*area/(dx^2 rho) of an open face that
     // is not area = rho = 1, the flux area*u/dx of a face with 0 < area and
-    // not (area = 1 with dx a power of two)
+    // not (area = 1 with dx a power of two); the fluxes of 3D faces with area 1
+    // only next to a fluid cell
     double *w[3];
     double *q[3];
 };

@@ -100,6 +100,11 @@ struct FaceParams {
     // dt for the velocity update's dt dp / dx by integer instructions
     // (gbp_exact.cuh), with 1/dx as its power of two
     MulConst dt_mul;
+    // dt / dx as a float pair (the velocity update), 1/dx for the fluxes when
+    // dx is no power of two (both gbp_exact.cuh)
+    PairConst dt_dx;
+    RecipConst by_dx;
+    int div_ok;  // |dt| and dx in [2^-160, 2^160]
 };
 
 // a[n] for n in [0, 7) by selects (an indexed kernel parameter would be
@@ -135,6 +140,15 @@ __device__ __noinline__ double face_weight_fp64(double dt, float area, float rho
 __device__ __noinline__ double face_flux_fp64(float area, float uf, double dx, int dx_pow2, double inv_dx) {
     const double x = (double)area * (double)uf;
     return dx_pow2 ? x * inv_dx : x / dx;
+}
+
+// u/dx of a face with area 1 (dx not a power of two), not inlined so that its
+// FP64 instructions are never issued predicated off.
+__device__ __noinline__ double unit_flux_fp64(float uf, const RecipConst by_dx, int in_range) {
+    const int ex = (int)(__float_as_uint(uf) >> 23 & 0xffu);
+    // (inf, NaN, or a dx outside div_round's range)
+    if (ex == 255 || !in_range) return (double)uf / by_dx.d;
+    return div_round(by_dx, f2d_exact(uf));
 }
 
 // face_area of an interior 3D face from its four corner levels (q00, q10,
@@ -505,12 +519,12 @@ __global__ void __launch_bounds__(BLOCK_THREADS) velocity_kernel(Grid g, double 
 // warp instruction costs its pipe slots however few lanes it has. The 3D
 // kernel therefore queues them in shared memory and computes them
 // together, a full warp at a time, when the queue fills and at the end.
-constexpr int FACE_QUEUE = 1024;
+// Entries are the face's node and direction; its values are gathered again.
+constexpr int FACE_QUEUE = 4096, FACE_ROUNDS = 4;
+static_assert(FACE_QUEUE >= 3 * BLOCK_THREADS * FACE_ROUNDS + 1024, "room for the faces of FACE_ROUNDS nodes a thread");
 struct FaceQueue {
-    long long f[FACE_QUEUE];
-    float q[4][FACE_QUEUE];  // the square's corners (area3's order)
-    float fa[FACE_QUEUE], fb[FACE_QUEUE], uf[FACE_QUEUE];
-    unsigned char tag[FACE_QUEUE];  // d | interior << 2
+    unsigned node[FACE_QUEUE];
+    unsigned char d[FACE_QUEUE];
 };
 
 // area3 needs area3_fp64 (corners neither all >= 0 with eps_solid <= 1
@@ -525,7 +539,13 @@ __device__ __forceinline__ bool rho_slow(float f0, float f1, const FaceParams &f
     return (f0 < 0.0f || f1 < 0.0f) && !fp.eps_fluid_le1;
 }
 
-template <int DIM>
+// POW2: dx is a power of two (the fluxes of faces with area 1 are formed by
+// the cell pass, and u, v, w are read for cut faces alone).
+// Node, cell and face indices fit 32 bits (node_coords), and are formed
+// without 64-bit products: these passes are bound by integer instructions.
+// 256^3 (dx = 2^-8): 411 -> 175 us; the 64 grids of a batch, 32^3 to 160^3,
+// most with dx no power of two: 105 -> 41 us each on average.
+template <int DIM, bool POW2>
 __global__ void __launch_bounds__(BLOCK_THREADS) faces_kernel(Grid g, double dt, double dx, FaceParams fp,
                                                               const float *__restrict__ solid,
                                                               const float *__restrict__ fluid,
@@ -535,9 +555,8 @@ __global__ void __launch_bounds__(BLOCK_THREADS) faces_kernel(Grid g, double dt,
     const long long NX = g.nx + 1, NY = g.ny + 1, NZ = g.dim == 3 ? g.nz + 1 : 1;
     const long long total = NX * NY * NZ;
     const float *vel[3] = {u, v, w};
-    const int n[3] = {g.nx, g.ny, g.nz};
     // One face's outputs from its fractions and velocity.
-    auto emit = [&](int d, long long f, float area, float rho, float uf) {
+    auto emit = [&](int d, unsigned f, float area, float rho, float uf) {
         const bool open = area && rho;
         fa.rho[d][f] = open ? rho : (area ? -1.0f : 0.0f);
         fa.area[d][f] = area;
@@ -546,101 +565,110 @@ __global__ void __launch_bounds__(BLOCK_THREADS) faces_kernel(Grid g, double dt,
             fa.w[d][f] = face_weight_fp64(dt, area, rho, dx, fp.dx_pow2, fp.inv_dx2);
         if (area != 0.0f && !(area == 1.0f && fp.dx_pow2)) fa.q[d][f] = face_flux_fp64(area, uf, dx, fp.dx_pow2, fp.inv_dx);
     };
+    if constexpr (DIM == 2) {
+        const int n[2] = {g.nx, g.ny};
+        for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total;
+             t += (long long)gridDim.x * blockDim.x) {
+            int i, j, k;
+            node_coords(g, t, i, j, k);
+            const int pi[2] = {i, j};
+            for (int d = 0; d < 2; ++d) {
+                if (pi[1 - d] >= n[1 - d]) continue;
+                const unsigned f = (unsigned)face_index(g, d, i, j, k);
+                emit(d, f, face_area(g, solid, d, i, j, k, fp), face_rho(g, fluid, d, i, j, k, fp, 1),
+                     __ldg(vel[d] + f));
+            }
+        }
+        return;
+    }
     __shared__ FaceQueue Q;
     __shared__ int qn;
     if (threadIdx.x == 0) qn = 0;
     __syncthreads();
+    const unsigned nx = (unsigned)g.nx, ny = (unsigned)g.ny, nxy = nx * ny, sx = nx + 1, sxy = sx * (ny + 1);
     // the queued faces, a thread each; the fractions by the same functions
     // the direct path uses
     auto flush = [&]() {
         __syncthreads();
         const int cnt = qn;
         for (int e = threadIdx.x; e < cnt; e += blockDim.x) {
-            const int d = Q.tag[e] & 3;
-            const float area = (Q.tag[e] >> 2) ? area3(Q.q[0][e], Q.q[1][e], Q.q[2][e], Q.q[3][e], fp) : 0.0f;
-            emit(d, Q.f[e], area, rho_of(Q.fa[e], Q.fb[e], fp), Q.uf[e]);
+            const unsigned t = Q.node[e];
+            const int d = Q.d[e];
+            int i, j, k;
+            node_coords(g, t, i, j, k);
+            // interior faces alone are queued: their cells are (i, j, k) and the one before
+            const unsigned c = (unsigned)i + nx * ((unsigned)j + ny * (unsigned)k);
+            const unsigned fi = d == 0 ? (unsigned)i + sx * ((unsigned)j + ny * (unsigned)k)
+                                       : (d == 1 ? c + nx * (unsigned)k : c);
+            const unsigned o1 = d == 0 ? sx : 1u, o3 = d == 2 ? sx : sxy;
+            const float area = area3(__ldg(solid + t), __ldg(solid + (t + o1)), __ldg(solid + (t + o1 + o3)),
+                                     __ldg(solid + (t + o3)), fp);
+            const float fA = __ldg(fluid + c), fB = __ldg(fluid + (c - (d == 0 ? 1u : (d == 1 ? nx : nxy))));
+            emit(d, fi, area, rho_of(fA, fB, fp), __ldg(vel[d] + fi));
         }
         __syncthreads();
         if (threadIdx.x == 0) qn = 0;
         __syncthreads();
     };
     // block-uniform trip count (the queue's flushes are block-wide)
+    int round = 0;
     for (long long base = (long long)blockIdx.x * blockDim.x; base < total; base += (long long)gridDim.x * blockDim.x) {
-        const long long t = base + threadIdx.x;
-        // room for this iteration's faces (at most 3 per thread): the barrier's
-        // OR includes the last pusher's own reading, which is the count
-        if (DIM == 3 && __syncthreads_or(qn > FACE_QUEUE - 3 * BLOCK_THREADS)) flush();
-        if (t >= total) continue;
+        // room for the next FACE_ROUNDS nodes' faces (at most 3 each): the
+        // barrier's OR includes the last pusher's own reading, which is the count
+        if (round++ == FACE_ROUNDS) {
+            if (__syncthreads_or(qn > FACE_QUEUE - 3 * BLOCK_THREADS * FACE_ROUNDS)) flush();
+            round = 1;
+        }
+        if (base + threadIdx.x >= total) continue;
+        const unsigned t = (unsigned)(base + threadIdx.x);
         int i, j, k;
         node_coords(g, t, i, j, k);
-        if constexpr (DIM == 3) {
-            // The node's three faces with every load issued first (the
-            // per-face form waits for each face's loads in turn: its stores
-            // could alias the next face's inputs). A face exists when its
-            // other two indices are cells; its area comes from its corners
-            // unless it lies on the domain boundary (area 0).
-            const bool ci = i < g.nx, cj = j < g.ny, ck = k < g.nz;
-            const bool ex[3] = {cj && ck, ci && ck, ci && cj};
-            const bool in[3] = {ex[0] && i > 0 && ci, ex[1] && j > 0 && cj, ex[2] && k > 0 && ck};
-            const long long sx = NX, sxy = NX * NY;
-            const float *s0 = solid + i + sx * j + sxy * k;
-            const float S000 = (in[0] || in[1] || in[2]) ? __ldg(s0) : 0.0f;
-            const float S010 = (in[0] || in[2]) ? __ldg(s0 + sx) : 0.0f;
-            const float S001 = (in[0] || in[1]) ? __ldg(s0 + sxy) : 0.0f;
-            const float S011 = in[0] ? __ldg(s0 + sx + sxy) : 0.0f;
-            const float S100 = (in[1] || in[2]) ? __ldg(s0 + 1) : 0.0f;
-            const float S101 = in[1] ? __ldg(s0 + 1 + sxy) : 0.0f;
-            const float S110 = in[2] ? __ldg(s0 + 1 + sx) : 0.0f;
-            // the face's cells, clamped as face_rho clamps them
-            const int a0 = min(i, g.nx - 1), a1 = min(j, g.ny - 1), a2 = min(k, g.nz - 1);
-            const long long ca = cell_index(g, a0, a1, a2);
-            const bool any = ex[0] || ex[1] || ex[2];
-            const float fA = any ? __ldg(fluid + ca) : 0.0f;
-            const float fB0 = ex[0] ? __ldg(fluid + cell_index(g, min(max(i - 1, 0), g.nx - 1), a1, a2)) : 0.0f;
-            const float fB1 = ex[1] ? __ldg(fluid + cell_index(g, a0, min(max(j - 1, 0), g.ny - 1), a2)) : 0.0f;
-            const float fB2 = ex[2] ? __ldg(fluid + cell_index(g, a0, a1, min(max(k - 1, 0), g.nz - 1))) : 0.0f;
-            long long f[3];
-            float uf[3];
+        // The node's three faces, every load first. A face exists when its
+        // other two indices are cells; its area comes from its corners unless
+        // it lies on the domain boundary (area 0).
+        const bool ci = i < g.nx, cj = j < g.ny, ck = k < g.nz;
+        const bool ex[3] = {cj && ck, ci && ck, ci && cj};
+        const bool in[3] = {ex[0] && i > 0 && ci, ex[1] && j > 0 && cj, ex[2] && k > 0 && ck};
+        const bool any = in[0] || in[1] || in[2];
+        const unsigned c = (unsigned)i + nx * ((unsigned)j + ny * (unsigned)k);
+        const unsigned f[3] = {c + ((unsigned)j + ny * (unsigned)k), c + nx * (unsigned)k, c};
+        const float S000 = any ? __ldg(solid + t) : 0.0f;
+        const float S010 = in[0] || in[2] ? __ldg(solid + (t + sx)) : 0.0f;
+        const float S001 = in[0] || in[1] ? __ldg(solid + (t + sxy)) : 0.0f;
+        const float S011 = in[0] ? __ldg(solid + (t + sx + sxy)) : 0.0f;
+        const float S100 = in[1] || in[2] ? __ldg(solid + (t + 1u)) : 0.0f;
+        const float S101 = in[1] ? __ldg(solid + (t + 1u + sxy)) : 0.0f;
+        const float S110 = in[2] ? __ldg(solid + (t + 1u + sx)) : 0.0f;
+        const float fA = any ? __ldg(fluid + c) : 0.0f;
+        const float fB[3] = {in[0] ? __ldg(fluid + (c - 1u)) : 0.0f, in[1] ? __ldg(fluid + (c - nx)) : 0.0f,
+                             in[2] ? __ldg(fluid + (c - nxy)) : 0.0f};
+        float uf[3];
 #pragma unroll
-            for (int d = 0; d < 3; ++d) {
-                f[d] = face_index(g, d, i, j, k);
-                uf[d] = ex[d] ? __ldg(vel[d] + f[d]) : 0.0f;
+        for (int d = 0; d < 3; ++d) uf[d] = !POW2 && in[d] ? __ldg(vel[d] + f[d]) : 0.0f;
+        // fractions of 0 or 1 here; a face that needs the FP64 forms is queued
+        auto face = [&](int d, float q00, float q10, float q11, float q01) {
+            if (!in[d]) {
+                fa.rho[d][f[d]] = 0.0f;
+                fa.area[d][f[d]] = 0.0f;
+                return;
             }
-            // fractions of 0 or 1 here; a face that needs the FP64 forms is
-            // queued with its inputs
-            auto face = [&](int d, float q00, float q10, float q11, float q01, float fB) {
-                if (in[d] ? area3_slow(q00, q10, q11, q01, fp) || rho_slow(fA, fB, fp) : rho_slow(fA, fB, fp)) {
-                    const int e = atomicAdd(&qn, 1);
-                    Q.f[e] = f[d];
-                    Q.q[0][e] = q00;
-                    Q.q[1][e] = q10;
-                    Q.q[2][e] = q11;
-                    Q.q[3][e] = q01;
-                    Q.fa[e] = fA;
-                    Q.fb[e] = fB;
-                    Q.uf[e] = uf[d];
-                    Q.tag[e] = (unsigned char)(d | (in[d] ? 4 : 0));
-                    return;
-                }
-                emit(d, f[d], in[d] ? area3(q00, q10, q11, q01, fp) : 0.0f, rho_of(fA, fB, fp), uf[d]);
-            };
-            if (ex[0]) face(0, S000, S010, S011, S001, fB0);
-            if (ex[1]) face(1, S000, S100, S101, S001, fB1);
-            if (ex[2]) face(2, S000, S100, S110, S010, fB2);
-        } else {
-            const int pi[3] = {i, j, k};
-            for (int d = 0; d < 2; ++d) {
-                bool exists = true;
-                for (int e = 0; e < 2; ++e)
-                    if (e != d && pi[e] >= n[e]) exists = false;
-                if (!exists) continue;
-                const long long f = face_index(g, d, i, j, k);
-                emit(d, f, face_area(g, solid, d, i, j, k, fp), face_rho(g, fluid, d, i, j, k, fp, 1),
-                     __ldg(vel[d] + f));
+            if (area3_slow(q00, q10, q11, q01, fp) || rho_slow(fA, fB[d], fp)) {
+                const int e = atomicAdd(&qn, 1);
+                Q.node[e] = t;
+                Q.d[e] = (unsigned char)d;
+                return;
             }
-        }
+            const bool open = q00 >= 0.0f, wet = fA < 0.0f || fB[d] < 0.0f;
+            fa.rho[d][f[d]] = open ? (wet ? 1.0f : -1.0f) : 0.0f;
+            fa.area[d][f[d]] = open ? 1.0f : 0.0f;
+            // (a flux that no cell's right-hand side reads is not formed)
+            if (!POW2 && open && wet) fa.q[d][f[d]] = unit_flux_fp64(uf[d], fp.by_dx, fp.div_ok);
+        };
+        if (ex[0]) face(0, S000, S010, S011, S001);
+        if (ex[1]) face(1, S000, S100, S101, S001);
+        if (ex[2]) face(2, S000, S100, S110, S010);
     }
-    if (DIM == 3) flush();
+    flush();
 }
 
 // The FP64 fallbacks of the cell pass, out of line (see faces_kernel):
@@ -689,8 +717,10 @@ __device__ __noinline__ double recip_fp64(double a) { return 1.0 / a; }
 // template argument, so that no FP64 addition is issued predicated off).
 // Four blocks per SM (64 registers, a few spilled): the pass is bound by
 // instruction issue, and more warps measured 40 us faster at 256^3 than
-// three blocks at 80 registers.
-template <bool RC>
+// three blocks at 80 registers. POW2 as in faces_kernel; without it the
+// right-hand side is the sum of the stored fluxes, which were gathered by a
+// loop out of line: the batch's grids 105 -> 64 us.
+template <bool RC, bool POW2>
 __global__ void __launch_bounds__(BLOCK_THREADS, 4) assemble_faces_kernel(
     Grid g, double dt, double dx, FaceParams fp, double rhs_correct, const float *__restrict__ fluid,
     const float *__restrict__ u, const float *__restrict__ v, const float *__restrict__ w, FaceArrays fa,
@@ -710,7 +740,8 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 4) assemble_faces_kernel(
         for (int kk = 0; kk < g.tz; ++kk) {
             const int k = k0 + kk;
             if (k >= g.nz) break;
-            const long long c = cell_index(g, i, j, k);
+            const unsigned row = (unsigned)j + (unsigned)g.ny * (unsigned)k;
+            const unsigned c = (unsigned)i + (unsigned)g.nx * row;
             double dg = 0.0, rhs = 0.0, cpl[3] = {0.0, 0.0, 0.0};
             bool unknown = false, unit = true;
             int nopen = 0;
@@ -724,13 +755,9 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 4) assemble_faces_kernel(
             // the index of face nq from the cell's: the -x face of cell c is
             // c + j + ny k, the -y face c + nx k, the -z face c; the + faces
             // one step further (face_index, without its multiplications)
-            auto findex = [&](int nq) {
-                const int d = nq >> 1;
-                const long long base = c + (d == 0 ? (long long)j + (long long)g.ny * k
-                                                   : (d == 1 ? (long long)g.nx * k : 0ll));
-                const long long step = d == 0 ? 1ll : (d == 1 ? (long long)g.nx : (long long)g.nx * g.ny);
-                return (nq & 1) == 0 ? base + step : base;
-            };
+            const unsigned step[3] = {1u, (unsigned)g.nx, (unsigned)g.nx * (unsigned)g.ny};
+            const unsigned low[3] = {c + row, c + (unsigned)g.nx * (unsigned)k, c};
+            auto findex = [&](int nq) { return (nq & 1) == 0 ? low[nq >> 1] + step[nq >> 1] : low[nq >> 1]; };
 #pragma unroll
             for (int nq = 0; nq < 6; ++nq) {
                 const int d = nq >> 1;
@@ -738,11 +765,11 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 4) assemble_faces_kernel(
                 int q[3] = {i, j, k};
                 q[d] += plus ? 1 : -1;
                 has[nq] = d < g.dim && q[d] >= 0 && q[d] < n[d];
-                const long long fi = has[nq] ? findex(nq) : 0;
+                const unsigned fi = findex(nq);
                 fr[nq] = has[nq] ? __ldg(fa.rho[d] + fi) : 0.0f;
                 ar[nq] = has[nq] ? __ldg(fa.area[d] + fi) : 0.0f;
-                uv[nq] = has[nq] ? __ldg(vel[d] + fi) : 0.0f;
-                fq[nq] = has[nq] ? __ldg(fluid + cell_index(g, q[0], q[1], q[2])) : 0.0f;
+                uv[nq] = POW2 && has[nq] ? __ldg(vel[d] + fi) : 0.0f;
+                fq[nq] = has[nq] ? __ldg(fluid + (plus ? c + step[d] : c - step[d])) : 0.0f;
             }
             // the weight of an open face
             auto wface = [&](int nq) {
@@ -753,7 +780,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 4) assemble_faces_kernel(
                 // the right-hand side's terms -+u/dx by face (0 where a face
                 // has no term or area 0: adding +-0 changes no sum)
                 float terms[6] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
-                bool qexact = fp.dx_pow2 != 0;
+                bool qexact = POW2;
 #pragma unroll
                 for (int nq = 0; nq < 6; ++nq) {
                     if (!has[nq]) continue;
@@ -770,8 +797,17 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 4) assemble_faces_kernel(
                 }
                 if (unknown) {
                     dg = unit ? pick7(fp.w_sum, nopen) : diag_fp64(g, fa, i, j, k, fp.w_unit);
+                    if constexpr (!POW2) {
+                        // the stored fluxes, every load first; a face that is
+                        // not there adds a zero, which changes no sum
+                        double qv[6];
+#pragma unroll
+                        for (int nq = 0; nq < 6; ++nq) qv[nq] = ar[nq] != 0.0f ? __ldg(fa.q[nq >> 1] + findex(nq)) : 0.0;
+#pragma unroll
+                        for (int nq = 0; nq < 6; ++nq) rhs = (nq & 1) == 0 ? rhs - qv[nq] : rhs + qv[nq];
+                    }
                     // 0x15: the + faces' terms are negated
-                    if (!(qexact && exact_sum(terms, 6, 0x15u, fp.inv_dx_exp, rhs)))
+                    else if (!(qexact && exact_sum(terms, 6, 0x15u, fp.inv_dx_exp, rhs)))
                         rhs = rhs_fp64(g, fa, u, v, w, i, j, k, fp.dx_pow2, fp.inv_dx);
                 }
             }
@@ -846,6 +882,19 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 4) assemble_faces_kernel(
     }
 }
 
+// The FP64 evaluation of face_update, out of line (see faces_kernel).
+__device__ __noinline__ float update_fp64(float dp, float rho, double dt, double dx, const FaceParams &fp) {
+    float vv;
+    if (rho == 1.0f) {
+        if (mul_round(fp.dt_mul, dp, vv)) return vv;
+        const int ex = (int)(__float_as_uint(dp) >> 23 & 0xffu);
+        // in div_round's range: dp normal, dt and dx within 2^160
+        if (!fp.dx_pow2 && fp.div_ok && ex != 0 && ex != 255) return d2f_rn(div_round(fp.by_dx, dt * f2d_exact(dp)));
+        return (float)div_dx(dt * (double)dp, dx, fp);
+    }
+    return (float)(dt * (double)dp / ((double)rho * dx));
+}
+
 // The new velocity of one face from its stored fraction (fr), the pressures
 // on its two sides and its velocity; interior: not on the domain boundary.
 // Open faces get u - (float)(dt (pc - pm) / (rho dx)), every other face 0.
@@ -855,19 +904,21 @@ __device__ __forceinline__ float face_update(float fr, bool interior, float pc, 
     const float rho = fluid_exists ? fr : 1.0f;
     if (!open || !interior) return 0.0f;
     const float dp = pc - pm;
-    // rho * dx == dx exactly when rho == 1; (float)(dt dp / dx) by integer
-    // instructions where they decide (gbp_exact.cuh)
     float vv;
-    if (rho == 1.0f && mul_round(fp.dt_mul, dp, vv)) return uf - vv;
-    const double val = rho == 1.0f ? div_dx(dt * (double)dp, dx, fp) : dt * (double)dp / ((double)rho * dx);
-    return uf - (float)val;
+    // by float pairs where they decide (gbp_exact.cuh)
+    if (!quot_round(fp.dt_dx, dp, rho, vv)) vv = update_fp64(dp, rho, dt, dx, fp);
+    return uf - vv;
 }
 
 // Velocity update from the stored face fractions (same rule as
 // velocity_kernel): open faces inside the domain get the pressure gradient,
 // every other face 0; with no fluid anywhere every face with area > 0 is open
-// with rho = 1 (macutility3.cpp:190-192).
-__global__ void __launch_bounds__(BLOCK_THREADS) velocity_faces_kernel(Grid g, double dt, double dx, FaceParams fp,
+// with rho = 1 (macutility3.cpp:190-192). Bound by instructions: the quotients
+// by float pairs instead of 64-bit integer products (dx a power of two) or
+// FP64 divisions (any other dx), 32-bit indices. 256^3 (dx = 2^-8): 317 ->
+// 205 us; the batch's grids (see faces_kernel): 52 -> 18 us.
+__global__ void __launch_bounds__(BLOCK_THREADS) velocity_faces_kernel(Grid g, double dt, double dx,
+                                                                       const __grid_constant__ FaceParams fp,
                                                                        const float *__restrict__ p, FaceArrays fa,
                                                                        float *__restrict__ u, float *__restrict__ v,
                                                                        float *__restrict__ w,
@@ -876,38 +927,30 @@ __global__ void __launch_bounds__(BLOCK_THREADS) velocity_faces_kernel(Grid g, d
     const long long NX = g.nx + 1, NY = g.ny + 1, NZ = g.dim == 3 ? g.nz + 1 : 1;
     const long long total = NX * NY * NZ;
     float *vel[3] = {u, v, w};
-    const int n[3] = {g.nx, g.ny, g.nz};
-    auto update = [&](float fr, bool interior, float pc, float pm, float uf) {
-        return face_update(fr, interior, pc, pm, uf, fluid_exists, dt, dx, fp);
-    };
+    const unsigned nx = (unsigned)g.nx, ny = (unsigned)g.ny;
+    const unsigned back[3] = {1u, nx, nx * ny};
     for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total;
          t += (long long)gridDim.x * blockDim.x) {
         int i, j, k;
         node_coords(g, t, i, j, k);
-        const int pi[3] = {i, j, k};
-        bool ex[3], in[3];
-        long long f[3];
+        const bool ci = i < g.nx, cj = j < g.ny, ck = g.dim == 2 || k < g.nz;
+        const bool ex[3] = {cj && ck, ci && ck, g.dim == 3 && ci && cj};
+        const bool in[3] = {ex[0] && i > 0 && ci, ex[1] && j > 0 && cj, ex[2] && k > 0 && ck};
+        const unsigned c = (unsigned)i + nx * ((unsigned)j + ny * (unsigned)k);
+        const unsigned f[3] = {c + ((unsigned)j + ny * (unsigned)k), c + nx * (unsigned)k, c};
         float fr[3], pm[3], uf[3];
-        bool any_in = false;
         // every load of the node's faces first, then the updates (the
         // per-face form waits for each face's loads in turn)
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
-            ex[d] = d < g.dim;
-#pragma unroll
-            for (int e = 0; e < 3; ++e)
-                if (e < g.dim && e != d && pi[e] >= n[e]) ex[d] = false;
-            in[d] = ex[d] && pi[d] > 0 && pi[d] < n[d];
-            any_in = any_in || in[d];
-            f[d] = ex[d] ? face_index(g, d, i, j, k) : 0;
-            fr[d] = ex[d] ? __ldg(fa.rho[d] + f[d]) : 0.0f;
+            fr[d] = in[d] ? __ldg(fa.rho[d] + f[d]) : 0.0f;
             uf[d] = in[d] ? vel[d][f[d]] : 0.0f;
-            pm[d] = in[d] ? __ldg(p + cell_index(g, i - (d == 0), j - (d == 1), k - (d == 2))) : 0.0f;
+            pm[d] = in[d] ? __ldg(p + (c - back[d])) : 0.0f;
         }
-        const float pc = any_in ? __ldg(p + cell_index(g, i, j, k)) : 0.0f;
+        const float pc = in[0] || in[1] || in[2] ? __ldg(p + c) : 0.0f;
 #pragma unroll
         for (int d = 0; d < 3; ++d)
-            if (ex[d]) vel[d][f[d]] = update(fr[d], in[d], pc, pm[d], uf[d]);
+            if (ex[d]) vel[d][f[d]] = face_update(fr[d], in[d], pc, pm[d], uf[d], fluid_exists, dt, dx, fp);
     }
 }
 
@@ -997,6 +1040,9 @@ FaceParams face_params(const SetupParams &sp, double dx, double dt) {
     fp.unit_lo = split_lo(fp.w_unit, fp.unit_hi);
     fp.dt_mul = make_mul_const(dt, fp.dx_pow2 ? fp.inv_dx_exp : 0);
     fp.dt_mul.ok = fp.dt_mul.ok && fp.dx_pow2;
+    fp.dt_dx = make_pair_const(dt / dx);
+    fp.by_dx = make_recip_const(dx);
+    fp.div_ok = std::fabs(dt) >= 6.9e-49 && std::fabs(dt) <= 1.4e48 && dx >= 6.9e-49 && dx <= 1.4e48;
     return fp;
 }
 
@@ -1035,10 +1081,11 @@ cudaError_t launch_faces(const Grid &g, double dt, double dx, const SetupParams 
                          int grid_blocks, cudaStream_t stream) {
     const FaceParams fp = face_params(sp, dx, dt);
     if (g.dim == 3)
-        faces_kernel<3><<<node_blocks(g, grid_blocks), BLOCK_THREADS, 0, stream>>>(g, dt, dx, fp, solid, fluid, u, v, w,
+        (fp.dx_pow2 ? faces_kernel<3, true> : faces_kernel<3, false>)
+            <<<node_blocks(g, grid_blocks), BLOCK_THREADS, 0, stream>>>(g, dt, dx, fp, solid, fluid, u, v, w,
                                                                                    fa);
     else
-        faces_kernel<2><<<node_blocks(g, grid_blocks), BLOCK_THREADS, 0, stream>>>(g, dt, dx, fp, solid, fluid, u, v, w,
+        faces_kernel<2, false><<<node_blocks(g, grid_blocks), BLOCK_THREADS, 0, stream>>>(g, dt, dx, fp, solid, fluid, u, v, w,
                                                                                    fa);
     return cudaGetLastError();
 }
@@ -1050,14 +1097,11 @@ cudaError_t launch_assemble_faces(const Grid &g, double dt, double dx, const Set
     const FaceParams fp = face_params(sp, dx, dt);
     int blocks = (int)(g.ntiles < grid_blocks ? g.ntiles : grid_blocks);
     if (blocks < 1) blocks = 1;
-    if (sp.rhs_correct != 0.0)
-        assemble_faces_kernel<true><<<blocks, BLOCK_THREADS, 0, stream>>>(
-            g, dt, dx, fp, sp.rhs_correct, fluid, u, v, g.dim == 3 ? w : v, fa, diag, cx, cy, g.dim == 3 ? cz : cy, b, o,
-            sc);
-    else
-        assemble_faces_kernel<false><<<blocks, BLOCK_THREADS, 0, stream>>>(
-            g, dt, dx, fp, sp.rhs_correct, fluid, u, v, g.dim == 3 ? w : v, fa, diag, cx, cy, g.dim == 3 ? cz : cy, b, o,
-            sc);
+    const auto kernel = sp.rhs_correct != 0.0
+                            ? (fp.dx_pow2 ? assemble_faces_kernel<true, true> : assemble_faces_kernel<true, false>)
+                            : (fp.dx_pow2 ? assemble_faces_kernel<false, true> : assemble_faces_kernel<false, false>);
+    kernel<<<blocks, BLOCK_THREADS, 0, stream>>>(g, dt, dx, fp, sp.rhs_correct, fluid, u, v, g.dim == 3 ? w : v, fa, diag,
+                                                 cx, cy, g.dim == 3 ? cz : cy, b, o, sc);
     return cudaGetLastError();
 }
 
