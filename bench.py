@@ -428,7 +428,7 @@ def run_gbp(args):
     # per iteration; the slowest is the dominant one
     if args.solver == "mgpcg":
         kernels = {10: "presmooth_kernel", 12: "restrict_kernel", 13: "post_black_kernel",
-                   14: "red_dot_kernel", 15: "direction_kernel", 16: "spmv_kernel", 17: "update_kernel"}
+                   14: "red_dot_kernel", 16: "direction_spmv_kernel", 17: "update_kernel"}
     else:
         kernels = {0: "cg_spmv_kernel", 1: "cg_update_kernel", 2: "cg_direction_kernel"}
     timed = {}
@@ -830,7 +830,7 @@ def run_gbp_advect(args):
                      "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s", "frac": round(achieved / peak, 4),
                      "traffic": committed_traffic(args.workload, "face_passes"), "peak_source": peak_kind,
                      "algorithmic_bytes_per_launch": face_bytes_alg, "ms_per_launch": round(face_ms, 5),
-                     "limiter": "FP64 pipe: the reference's double-precision traces and trilinear weights",
+                     "limiter": "instruction issue: float-pair traces and trilinear weights (the FP64 form decides where their rounding test cannot)",
                      "kernels": {"face_passes": {"ms": round(face_ms, 5),
                                                  "GBps": round(face_bytes_alg / (face_ms * 1e-3) / 1e9, 1)},
                                  "cell_passes": {"ms": round(cell_ms, 5),
