@@ -1,27 +1,29 @@
-// gbp_exact.cuh -- FP64 results of the setup's arithmetic from integer
-// instructions.
+// gbp_exact.cuh -- FP64 results of the setup's arithmetic without FP64
+// operations, or with few.
 //
 // On this GPU the FP64 pipe issues about two operations per clock per SM (a
-// sixty-fourth of the integer rate), and the assembly's FP64 sums and the
-// velocity update's FP64 products were bound by it. Where the operands allow,
-// the functions here produce the bit-identical double (or float) with
-// integer instructions and return true; otherwise they return false and the
-// caller evaluates the FP64 expression as before.
+// sixty-fourth of the integer rate). The functions here produce the
+// bit-identical double (or float) and return true, or return false, and the
+// caller evaluates the FP64 expression.
 //
 // * exact_sum: the sequential FP64 sum 0 + t_0 + t_1 + ... of terms
-//   t_i = f_i 2^k (floats f_i, one power of two; the face fluxes u/dx of the
-//   right-hand side when dx is a power of two). If every partial sum is a
+//   t_i = f_i 2^k (floats f_i, one power of two). If every partial sum is a
 //   double, no addition rounds and the result is the exact sum, which a
 //   64-bit integer holds when the terms' exponents span at most 36 binary
-//   orders. Both conditions are checked.
+//   orders. Both conditions are checked. (The assembly's right-hand side no
+//   longer takes it: six FP64 additions run beside the integer instructions
+//   that bound that pass.)
 // * mul_round: fl32(fl64(a f) 2^s) for a double a fixed per launch (dt) and
 //   a float f (a pressure difference): the 77-bit product of the
 //   significands rounded to 53 bits and then to 24, each to nearest with
 //   ties to even, as the two hardware roundings do; results outside the
 //   normal ranges take the FP64 path.
+// * quot_round: the same float, and that of a f / rho, from a float pair and
+//   a rounding test; div_round: x / d for a constant d in four operations.
 //
-// The same source compiles for the host (tests/test_kernel_host.py checks
-// both functions against the compiler's FP64 arithmetic).
+// The same source compiles for the host (tests/test_kernel_host.py and
+// tests/test_setup_quotients.py check the functions against the compiler's
+// FP64 arithmetic).
 #pragma once
 
 #include <cstring>

@@ -107,15 +107,6 @@ struct FaceParams {
     int div_ok;  // |dt| and dx in [2^-160, 2^160]
 };
 
-// a[n] for n in [0, 7) by selects (an indexed kernel parameter would be
-// copied to local memory)
-template <class T> __device__ __forceinline__ T pick7(const T (&a)[7], int n) {
-    T r = a[0];
-#pragma unroll
-    for (int q = 1; q < 7; ++q) r = n == q ? a[q] : r;
-    return r;
-}
-
 // x / dx, bit-identical either way (see FaceParams::dx_pow2)
 __device__ __forceinline__ double div_dx(double x, double dx, const FaceParams &fp) {
     return fp.dx_pow2 ? x * fp.inv_dx : x / dx;
@@ -504,8 +495,8 @@ __global__ void __launch_bounds__(BLOCK_THREADS) velocity_kernel(Grid g, double 
 // and flux area*u/dx. Pass 2, one thread per cell, forms its row from its
 // faces in the reference's order (+x, -x, +y, -y, +z, -z): weight w_unit on
 // faces with area = rho = 1, flux u 2^k when area = 1 and 1/dx = 2^k (an
-// exact double), and the sums in integers where they are exact
-// (gbp_exact.cuh), so diag, couplings and b are bit-identical to the
+// exact double, the factor applied to the sum), else the stored flux, so
+// diag, couplings and b are bit-identical to the
 // single-pass assemble_kernel (and to the reference); it also writes level 0
 // of the multigrid hierarchy (the FP32 operator of the mixed solver, or the
 // FP64 inverse diagonal) from the same registers.
@@ -719,7 +710,10 @@ __device__ __noinline__ double recip_fp64(double a) { return 1.0 / a; }
 // instruction issue, and more warps measured 40 us faster at 256^3 than
 // three blocks at 80 registers. POW2 as in faces_kernel; without it the
 // right-hand side is the sum of the stored fluxes, which were gathered by a
-// loop out of line: the batch's grids 105 -> 64 us.
+// loop out of line: the batch's grids 105 -> 64 us. With it the sums are FP64
+// additions, which run beside the integer instructions that bound the pass
+// (64-bit integer sums took about 200 a cell): 256^3 mixed 661 -> 592 us, FP64
+// 597 -> 515; the tables in shared memory before that 695 -> 661.
 template <bool RC, bool POW2>
 __global__ void __launch_bounds__(BLOCK_THREADS, 4) assemble_faces_kernel(
     Grid g, double dt, double dx, FaceParams fp, double rhs_correct, const float *__restrict__ fluid,
@@ -727,6 +721,19 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 4) assemble_faces_kernel(
     double *__restrict__ diag, double *__restrict__ cx, double *__restrict__ cy, double *__restrict__ cz,
     double *__restrict__ b, Level0Out o, Scalars *sc) {
     __shared__ unsigned long long sh_count[BLOCK_THREADS / 32];
+    // the tables by open faces: one or two shared loads a cell where selects
+    // over the kernel's parameters took seven instructions a table and word
+    __shared__ double sh_sum[7], sh_inv[7];
+    __shared__ float4 sh_f32[7];  // sum_hi, sum_lo, sum_inv
+    if (threadIdx.x == 0) {
+#pragma unroll
+        for (int q = 0; q < 7; ++q) {
+            sh_sum[q] = fp.w_sum[q];
+            sh_inv[q] = fp.inv_sum[q];
+            sh_f32[q] = make_float4(fp.sum_hi[q], fp.sum_lo[q], fp.sum_inv[q], 0.0f);
+        }
+    }
+    __syncthreads();
     const int tx = threadIdx.x & (TILE_X - 1), ty = threadIdx.x / TILE_X;
     unsigned long long my_count = 0;
     int my_fluid = 0;
@@ -796,7 +803,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 4) assemble_faces_kernel(
                     else if (ar[nq] != 0.0f) qexact = false;
                 }
                 if (unknown) {
-                    dg = unit ? pick7(fp.w_sum, nopen) : diag_fp64(g, fa, i, j, k, fp.w_unit);
+                    dg = unit ? sh_sum[nopen] : diag_fp64(g, fa, i, j, k, fp.w_unit);
                     if constexpr (!POW2) {
                         // the stored fluxes, every load first; a face that is
                         // not there adds a zero, which changes no sum
@@ -806,9 +813,17 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 4) assemble_faces_kernel(
 #pragma unroll
                         for (int nq = 0; nq < 6; ++nq) rhs = (nq & 1) == 0 ? rhs - qv[nq] : rhs + qv[nq];
                     }
-                    // 0x15: the + faces' terms are negated
-                    else if (!(qexact && exact_sum(terms, 6, 0x15u, fp.inv_dx_exp, rhs)))
+                    else if (qexact) {
+                        // the scaling by 1/dx, a power of two, commutes with the roundings
+#pragma unroll
+                        for (int nq = 0; nq < 6; ++nq) {
+                            const double t = f2d_exact(terms[nq]);
+                            rhs = (nq & 1) == 0 ? rhs - t : rhs + t;
+                        }
+                        rhs *= fp.inv_dx;
+                    } else {
                         rhs = rhs_fp64(g, fa, u, v, w, i, j, k, fp.dx_pow2, fp.inv_dx);
+                    }
                 }
             }
             if (unknown) {
@@ -831,9 +846,10 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 4) assemble_faces_kernel(
                 if (unit) {
                     // every open face unit (or no unknown: all zero): the
                     // conversions of the table values, computed on the host
-                    d32 = pick7(fp.sum_hi, nopen);
-                    dlo = pick7(fp.sum_lo, nopen);
-                    i32 = pick7(fp.sum_inv, nopen);
+                    const float4 tab = sh_f32[nopen];
+                    d32 = tab.x;
+                    dlo = tab.y;
+                    i32 = tab.z;
                     const bool bx = nonzero_bits(cpl[0]), by = nonzero_bits(cpl[1]), bz = nonzero_bits(cpl[2]);
                     x32 = bx ? fp.unit_hi : 0.0f;
                     xlo = bx ? fp.unit_lo : 0.0f;
@@ -866,7 +882,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 4) assemble_faces_kernel(
                     if (o.diag_lo) o.cz_lo[c] = zlo;
                 }
             }
-            if (o.inv64) o.inv64[c] = positive_bits(dg) ? (unit ? pick7(fp.inv_sum, nopen) : recip_fp64(dg)) : 0.0;
+            if (o.inv64) o.inv64[c] = positive_bits(dg) ? (unit ? sh_inv[nopen] : recip_fp64(dg)) : 0.0;
         }
     }
     unsigned long long wsum = my_count;
