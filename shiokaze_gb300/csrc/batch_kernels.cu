@@ -1766,7 +1766,8 @@ __global__ void __launch_bounds__(BLOCK_THREADS, OCC)
     update_kernel(const BLevel<T> *__restrict__ levels, const BSeg *__restrict__ segs, int nseg, int n,
                   const BScene<T> *__restrict__ scenes, int gate, double *part, int mode, BatchCounters *cnt,
                   const int *__restrict__ scene_of) {
-    if (batch_idle(cnt)) return;
+    // as in refine_residual_kernel: this launch lowers the counter
+    if (__syncthreads_or(threadIdx.x == 0 && batch_idle(cnt))) return;
     __shared__ double shf[BLOCK_THREADS / 32];
     __shared__ ItemCtx<T> ctx;
     reduce_items<T, MaxAcc<T>>(
@@ -1971,7 +1972,9 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 4) refine_residual_kernel(
     const BLevel<T> *__restrict__ levels, const BSeg *__restrict__ segs, int nseg, int n,
     const BScene<T> *__restrict__ scenes, double *part, int initial, double residual, int max_iter,
     double inner_rel, int inner_max, BatchCounters *cnt, const int *__restrict__ scene_of) {
-    if (!initial && *(const volatile int *)&cnt->refine <= 0) return;
+    // one thread decides for the block: the launch itself lowers the counter,
+    // and a block whose warps disagreed would copy half of a descriptor
+    if (!initial && !__syncthreads_or(threadIdx.x == 0 && *(const volatile int *)&cnt->refine > 0)) return;
     __shared__ double shf[BLOCK_THREADS / 32];
     __shared__ ItemCtx<T> ctx;
     reduce_items<T, MaxSumAcc<T>>(

@@ -279,6 +279,11 @@ template <class T> int BatchRunner::build(const BatchPlan<T> &plan, int grid_blo
     const int bucket = cells > 0 ? (int)std::lround(2.0 * std::log2((double)cells)) : 0;
     const std::string key = std::string(sizeof(T) == 4 ? "f" : "d") + std::to_string(bucket) +
                             (stage_mask_ ? "s" : "") + "/" + std::to_string(plan.nscenes > 1 ? 2 : 1);
+    // the tables and zeros went through the legacy stream, which does not order
+    // against the solve's (non-blocking) streams, and a copy from pageable
+    // memory may return before it has landed: a kernel that read a table too
+    // early would follow stray pointers
+    RUN_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
     if ((rc = tune_occupancy<T>(stream, key))) return rc;
     return GBP_OK;
 }

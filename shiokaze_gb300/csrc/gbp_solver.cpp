@@ -105,6 +105,7 @@ int Solver::prepare(const Grid &g, const gbp_params &p) {
     if (allocated_ && (g.nx != g_.nx || g.ny != g_.ny || g.nz != g_.nz || g.dim != g_.dim)) release();
     g_ = g;
     const size_t bytes = 8 * (size_t)g.ncell;
+    bool cleared = false;
     if (!allocated_) {
         double **bufs[] = {&st_.diag, &st_.cx, &st_.cy, &st_.cz, &st_.b, &st_.x, &st_.r, &st_.s, &st_.z};
         for (double **b : bufs) SOLVER_CUDA(cudaMalloc(b, bytes));
@@ -121,13 +122,18 @@ int Solver::prepare(const Grid &g, const gbp_params &p) {
             SOLVER_CUDA(cudaMalloc(&st_.faces.q[d], 8 * nf));
         }
         allocated_ = true;
+        cleared = true;
     }
     if (p.warm_start && !have_prev_buf_) {
         SOLVER_CUDA(cudaMalloc(&st_.prev, bytes));
         SOLVER_CUDA(cudaMemset(st_.prev, 0, bytes));
         have_prev_buf_ = true;
         st_.have_prev = false;
+        cleared = true;
     }
+    // the zeros above are written on the legacy stream, which does not order
+    // against the (non-blocking) streams of the solve
+    if (cleared) SOLVER_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
     if (p.solver == GBP_SOLVER_MGPCG) return prepare_mg(g, p);
     return GBP_OK;
 }
