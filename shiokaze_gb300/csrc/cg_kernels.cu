@@ -90,7 +90,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 6) cg_init_kernel(Grid g, Opera
             sc->iter = 0;
             sc->max_iter = max_iter;
             sc->alpha = sc->beta = 0.0;
-            if (res0 == 0.0) {  // pcg_solver.h:65-68
+            if (res0 == 0.0 && rho == rho) {  // pcg_solver.h:65-68
                 sc->done = 1;
                 sc->status = 1;
             } else if (rho == 0.0 || rho != rho) {  // :74-82
@@ -160,15 +160,16 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 6) cg_update_kernel(Grid g, dou
             sc->res = res;
             sc->r2 = rho_new;
             sc->iter += 1;
-            if (res <= sc->tol) {
+            // first, as |r|_inf passes over NaN
+            if (rho_new != rho_new || sc->alpha != sc->alpha) {
+                sc->done = 1;
+                sc->status = 3;
+            } else if (res <= sc->tol) {
                 sc->done = 1;
                 sc->status = 1;
             } else if (sc->iter >= sc->max_iter) {
                 sc->done = 1;
                 sc->status = 2;
-            } else if (rho_new != rho_new || sc->alpha != sc->alpha) {
-                sc->done = 1;
-                sc->status = 3;
             } else {
                 sc->beta = rho_new / sc->rho;
                 sc->rho = rho_new;

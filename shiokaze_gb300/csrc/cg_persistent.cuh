@@ -17,7 +17,7 @@
 // need not keep that shape does not: the stencil and the vector updates run
 // over the block's rows packed into full warps (of the 32 x 8 tiles of a
 // liquid many lanes have none), and the stop test is a flag, the sign bit of
-// the partial of r.r.
+// the partial of r.r (read only where r.r is no NaN).
 //
 // Exchange of the partials: a cluster's blocks push them into each other's
 // shared memory and meet at the hardware barrier; blocks of a cooperative
@@ -311,7 +311,8 @@ __global__ void __launch_bounds__(CLUSTER ? 512 : 768, 1) cg_persistent_kernel(c
         ++iter;
         if (tid == 0) {
             r2 = rho_new;
-            sh_status = !more ? 1 : (iter >= max_iter ? 2 : (rho_new != rho_new || alpha != alpha ? 3 : 0));
+            // NaN first: |r|_inf and the marks pass over it (a NaN's sign says nothing)
+            sh_status = rho_new != rho_new || alpha != alpha ? 3 : (!more ? 1 : (iter >= max_iter ? 2 : 0));
             sh_scalar = rho_new / rho;
             if (!sh_status) rho = rho_new;
         }

@@ -58,7 +58,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS) csr_init_kernel(long long n, co
             sc->iter = 0;
             sc->max_iter = max_iter;
             sc->alpha = sc->beta = 0.0;
-            if (res0 == 0.0) {  // pcg_solver.h:253-256
+            if (res0 == 0.0 && rho == rho) {  // pcg_solver.h:253-256
                 sc->done = 1;
                 sc->status = 1;
             } else if (rho == 0.0 || rho != rho) {  // :262-270
@@ -136,15 +136,16 @@ __global__ void __launch_bounds__(BLOCK_THREADS) csr_update_kernel(long long n, 
             sc->res = res;
             sc->r2 = rho_new;
             sc->iter += 1;
-            if (res <= sc->tol) {
+            // first, as |r|_inf passes over NaN
+            if (rho_new != rho_new || sc->alpha != sc->alpha) {
+                sc->done = 1;
+                sc->status = 3;
+            } else if (res <= sc->tol) {
                 sc->done = 1;
                 sc->status = 1;
             } else if (sc->iter >= sc->max_iter) {
                 sc->done = 1;
                 sc->status = 2;
-            } else if (rho_new != rho_new || sc->alpha != sc->alpha) {
-                sc->done = 1;
-                sc->status = 3;
             } else {
                 sc->beta = rho_new / sc->rho;
                 sc->rho = rho_new;
