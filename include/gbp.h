@@ -291,6 +291,17 @@ int gbp_debug_assemble(gbp_scene *scene, double dt, const float *solid, const fl
 #define GBP_WAIT_TILE 2
 int gbp_debug_fail_wait(gbp_scene *scene, int what, int block, int polls);
 
+/* Test hook for plain CG, in the scene's next solve with GBP_SOLVER_CG or,
+ * scene NULL, the context's next gbp_csr_cg. launched: nonzero takes the
+ * iterations as separate launches, as for systems too large for the one-launch
+ * form. steps > 0: iterations of one launch of that form (default 4096).
+ * polls > 0: its block `block` leaves out its arrivals and every wait polls at
+ * most `polls` times (1..2^22), so the other blocks' waits run out, they return
+ * and the solve returns GBP_ERR_CUDA (systems of up to 16384 rows or 64 tiles
+ * wait at a hardware barrier, which nothing runs out of). Nothing faults, and
+ * the next solve runs normally. No counterpart in the reference. */
+int gbp_debug_cg(gbp_ctx *ctx, gbp_scene *scene, int launched, int steps, int block, int polls);
+
 /* Benchmark hook: times `reps` back-to-back launches of one kernel on the
  * scene's last assembled system with CUDA events on `stream` (NULL = the
  * context's stream), after one untimed launch. which: GBP_KERNEL_*. Writes

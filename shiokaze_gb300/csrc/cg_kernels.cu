@@ -270,16 +270,16 @@ cudaError_t launch_cg_iteration(const Grid &g, Operator<double> A, double *x, do
     return cudaGetLastError();
 }
 
-bool cg_persistent_fits(const Grid &g, int grid_blocks) {
+bool cg_persistent_fits(const Grid &g, int grid_blocks, const CgDebug &debug) {
     const int nb = blocks_for(g, grid_blocks);
     const long long per = (g.ntiles + nb - 1) / nb * g.tz;
-    return g.ncell < (1LL << 31) && per <= 64 && cg_persistent_plan(nb, (int)per, grid_blocks / 6).use;
+    return g.ncell < (1LL << 31) && per <= 64 && cg_persistent_plan(nb, (int)per, grid_blocks / 6, debug).use;
 }
 
 cudaError_t launch_cg_persistent(const Grid &g, Operator<double> A, double *x, double *r, double *s, Scalars *sc,
-                                 Partials *pt, int grid_blocks, cudaStream_t stream) {
+                                 Partials *pt, int grid_blocks, const CgDebug &debug, cudaStream_t stream) {
     const int nb = blocks_for(g, grid_blocks);
-    CgPersistentPlan p = cg_persistent_plan(nb, (int)((g.ntiles + nb - 1) / nb * g.tz), grid_blocks / 6);
+    CgPersistentPlan p = cg_persistent_plan(nb, (int)((g.ntiles + nb - 1) / nb * g.tz), grid_blocks / 6, debug);
     p.args.x = x;
     p.args.r = r;
     p.args.s = s;

@@ -34,7 +34,8 @@
 // the L2 round trips.
 //
 // Waits: the cluster form uses the hardware barrier; the cooperative form
-// polls, bounded, and leaves with status 4 if a wait runs out.
+// polls, bounded (about two seconds), and leaves with status 4 if a wait runs
+// out (tests/test_gpu_cg_forms.py makes it).
 #pragma once
 
 #include "gbp_internal.cuh"
@@ -50,6 +51,7 @@ struct CgPersistentArgs {
     int sub;        // virtual blocks of a physical block
     int per_block;  // rows a thread has in one virtual block (the launched form's tiles and planes)
     int max_steps;  // iterations in this launch
+    int polls = 0, fail_block = 0;  // of CgDebug (the TEST form of the kernel)
 };
 
 #ifdef __CUDACC__
@@ -131,7 +133,9 @@ struct CsrRows {
 };
 
 // All blocks; false if a wait ran out. Writes before it are visible after it.
-template <bool CLUSTER> __device__ __forceinline__ bool meet(unsigned *count, unsigned &target) {
+// TEST: block a.fail_block leaves instead of arriving, waits poll a.polls times.
+template <bool CLUSTER, bool TEST>
+__device__ __forceinline__ bool meet(unsigned *count, unsigned &target, const CgPersistentArgs &a) {
     if (CLUSTER) {
         asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
         return true;
@@ -139,13 +143,15 @@ template <bool CLUSTER> __device__ __forceinline__ bool meet(unsigned *count, un
     target += gridDim.x;
     __syncthreads();
     int good = 1;
-    if (threadIdx.x == 0) {
+    if (TEST && (int)blockIdx.x == a.fail_block) {
+        good = 0;
+    } else if (threadIdx.x == 0) {
         asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(count) : "memory");
         unsigned seen;
         for (int it = 0;; ++it) {
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(count) : "memory");
             if (seen >= target) break;
-            if (it > kPolls) {
+            if (it > (TEST ? a.polls : kPolls)) {
                 good = 0;
                 break;
             }
@@ -154,11 +160,11 @@ template <bool CLUSTER> __device__ __forceinline__ bool meet(unsigned *count, un
     return __syncthreads_and(good) != 0;
 }
 
-template <class Rows, bool CLUSTER>
+template <class Rows, bool CLUSTER, bool TEST>
 __global__ void __launch_bounds__(CLUSTER ? 512 : 768, 1) cg_persistent_kernel(const Rows rows, const CgPersistentArgs a) {
     extern __shared__ double smem[];
     Scalars *sc = a.sc;
-    if (sc->done) return;
+    if (sc->done) return;  // (written after every block's last wait, so all threads read the same)
     const int T = blockDim.x, tid = threadIdx.x, nvb = a.sub, slots = nvb * a.per_block * 256;
     // home order: virtual block, item, thread
     double *R = smem, *S = R + slots, *Z = S + slots, *X = Z + slots;
@@ -223,7 +229,7 @@ __global__ void __launch_bounds__(CLUSTER ? 512 : 768, 1) cg_persistent_kernel(c
     const int max_iter = sc->max_iter;
     unsigned target = 0;
     unsigned *count = &sc->counter[4];
-    bool good = meet<CLUSTER>(count, target);
+    bool good = meet<CLUSTER, TEST>(count, target, a);
 
     // Every thread's items of the active virtual blocks, term by term in
     // order, then the trees: a partial per virtual block (negative if `large`)
@@ -260,7 +266,7 @@ __global__ void __launch_bounds__(CLUSTER ? 512 : 768, 1) cg_persistent_kernel(c
     // `marks` the partials are magnitudes and any tells whether one came
     // marked. False if a wait ran out.
     auto total = [&](double &sum, bool &any, const double *in, bool marks) {
-        if (!meet<CLUSTER>(count, target)) return false;
+        if (!meet<CLUSTER, TEST>(count, target, a)) return false;
         if (tid == 0) sh_large = 0;
         int marked = 0;
         if (tid < 256) {
@@ -327,7 +333,7 @@ __global__ void __launch_bounds__(CLUSTER ? 512 : 768, 1) cg_persistent_kernel(c
             S[h] = s;
             __stcg(a.s + cell[e], s);
         }
-        good = meet<CLUSTER>(count, target);
+        good = meet<CLUSTER, TEST>(count, target, a);
     }
     if (!good) status = 4;
     if (status < 4) {
@@ -340,7 +346,7 @@ __global__ void __launch_bounds__(CLUSTER ? 512 : 768, 1) cg_persistent_kernel(c
         }
         mx = warp_max_bits(mx);
         if (lane == 0 && mx) atomicMax(&sc->bits_max, mx);
-        if (!meet<CLUSTER>(count, target)) status = 4;
+        if (!meet<CLUSTER, TEST>(count, target, a)) status = 4;
     }
     if ((blockIdx.x == 0 || status == 4) && tid == 0) {
         if (status < 4) {
@@ -351,8 +357,10 @@ __global__ void __launch_bounds__(CLUSTER ? 512 : 768, 1) cg_persistent_kernel(c
             sc->res = __longlong_as_double((long long)__ldcg(&sc->bits_max));
             sc->iter = iter;
         }
+        // a run-out wait leaves done as it is: a block that starts only now
+        // must not find it set in some of its threads (it runs out too)
         sc->status = status;
-        sc->done = status != 0;
+        if (status < 4) sc->done = status != 0;
     }
 }
 
@@ -372,7 +380,7 @@ struct CgPersistentPlan {
     CgPersistentArgs args{};
 };
 
-inline CgPersistentPlan cg_persistent_plan(int nb, int per_block, int sms) {
+inline CgPersistentPlan cg_persistent_plan(int nb, int per_block, int sms, const CgDebug &debug = {}) {
     CgPersistentPlan p;
     p.cluster = nb <= 64;
     p.blocks = p.cluster ? 16 : (nb < sms ? nb : sms);
@@ -380,11 +388,13 @@ inline CgPersistentPlan cg_persistent_plan(int nb, int per_block, int sms) {
     p.args.sub = each;
     p.args.nb = nb;
     p.args.per_block = per_block;
-    p.args.max_steps = CG_PERSISTENT_STEPS;
+    p.args.max_steps = debug.steps > 0 ? debug.steps : CG_PERSISTENT_STEPS;
+    p.args.polls = debug.polls;
+    p.args.fail_block = debug.block;
     p.threads = p.cluster ? 512 : 768;
     const size_t slots = (size_t)each * per_block * 256;
     p.shared = slots * (4 * sizeof(double) + 2 * sizeof(int)) + (((size_t)each + 1) * TREE_PAD + 2 * 64) * sizeof(double);
-    p.use = p.shared <= 216 * 1024 && each <= 32 && nb <= MAX_GRID;
+    p.use = !debug.launched && p.shared <= 216 * 1024 && each <= 32 && nb <= MAX_GRID;
     return p;
 }
 
@@ -392,8 +402,9 @@ inline CgPersistentPlan cg_persistent_plan(int nb, int per_block, int sms) {
 // One launch of a planned solve on `stream`; sc->done tells whether it ended.
 template <class Rows>
 cudaError_t cg_persistent_launch(const CgPersistentPlan &p, const Rows &rows, cudaStream_t stream) {
-    const void *fn = p.cluster ? (const void *)cgp::cg_persistent_kernel<Rows, true>
-                               : (const void *)cgp::cg_persistent_kernel<Rows, false>;
+    const void *fn = p.cluster ? (const void *)cgp::cg_persistent_kernel<Rows, true, false>
+                     : p.args.polls > 0 ? (const void *)cgp::cg_persistent_kernel<Rows, false, true>
+                                        : (const void *)cgp::cg_persistent_kernel<Rows, false, false>;
     cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.shared);
     if (e == cudaSuccess && p.cluster) e = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     // the maximum, and the barrier's count

@@ -223,7 +223,7 @@ void csr_release(CsrWork &w) {
 }
 
 cudaError_t csr_cg_run(CsrWork &w, long long n, double residual, int max_iter, int grid_blocks,
-                       cudaStream_t stream, long long *launches) {
+                       const CgDebug &debug, cudaStream_t stream, long long *launches) {
     const int nb = blocks_for(n, grid_blocks);
     cudaError_t e;
     if ((e = cudaMemsetAsync(w.sc, 0, sizeof(Scalars), stream)) != cudaSuccess) return e;
@@ -232,22 +232,21 @@ cudaError_t csr_cg_run(CsrWork &w, long long n, double residual, int max_iter, i
     *launches += 1;
     const long long per = (n + (long long)nb * BLOCK_THREADS - 1) / ((long long)nb * BLOCK_THREADS);
     CgPersistentPlan plan;
-    if (per <= 64) plan = cg_persistent_plan(nb, (int)per, grid_blocks / 6);
+    if (per <= 64) plan = cg_persistent_plan(nb, (int)per, grid_blocks / 6, debug);
     if (plan.use) {
         plan.args.x = w.x;
         plan.args.r = w.r;
         plan.args.s = w.s;
         plan.args.sc = w.sc;
         plan.args.pt = w.pt;
-        for (int left = max_iter; e == cudaSuccess; left -= CG_PERSISTENT_STEPS) {
+        for (int left = max_iter; e == cudaSuccess; left -= plan.args.max_steps) {
             if ((e = cg_persistent_launch(plan, cgp::CsrRows{n, w.rowstart, w.cols, w.vals}, stream)) != cudaSuccess)
                 break;
             *launches += 1;
             if ((e = cudaMemcpyAsync(w.host_sc, w.sc, sizeof(Scalars), cudaMemcpyDeviceToHost, stream)) != cudaSuccess ||
                 (e = cudaStreamSynchronize(stream)) != cudaSuccess)
                 return e;
-            if (w.host_sc->status == 4) return cudaErrorLaunchTimeout;
-            if (w.host_sc->done || left <= 0) return cudaSuccess;
+            if (w.host_sc->done || w.host_sc->status == 4 || left <= 0) return cudaSuccess;
         }
         // blocks that cannot be resident together (a partitioned GPU): the launched form
         if (e != cudaErrorCooperativeLaunchTooLarge) return e;

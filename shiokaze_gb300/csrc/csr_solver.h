@@ -10,6 +10,7 @@
 #include <cuda_runtime.h>
 
 #include "gbp_internal.cuh"
+#include "gbp_kernels.h"
 
 namespace gbp {
 
@@ -32,8 +33,9 @@ void csr_release(CsrWork &w);
 // Runs the solve on w's arrays (rowstart, cols, vals and b filled for n
 // rows): x = 0, then iterations until the device reports done; host_sc
 // holds the final scalars (status 1 converged, 2 max iterations, 3
-// breakdown; res0, res, iter). *launches counts kernel launches.
+// breakdown, 4 a wait between blocks ran out; res0, res, iter). *launches
+// counts kernel launches.
 cudaError_t csr_cg_run(CsrWork &w, long long n, double residual, int max_iter, int grid_blocks,
-                       cudaStream_t stream, long long *launches);
+                       const CgDebug &debug, cudaStream_t stream, long long *launches);
 
 }  // namespace gbp

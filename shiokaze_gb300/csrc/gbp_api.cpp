@@ -76,6 +76,7 @@ struct gbp_ctx {
     cudaEvent_t ev_fork = nullptr, ev_side[kLanes - 1] = {};
     long long launches = 0;
     CsrWork csr;  // device arrays of gbp_csr_cg
+    CgDebug csr_debug;  // test hook gbp_debug_cg, for the next gbp_csr_cg
     AdvectWork adv;  // device scratch of gbp_advect3*
     // staging of the host-array advection call, grown on demand
     float *adv_stage = nullptr;
@@ -227,7 +228,10 @@ int gbp_csr_cg(gbp_ctx *c, long long n, const long long *rowstart, const long lo
     GBP_CUDA(cudaMemcpyAsync(w.b, b, sizeof(double) * (size_t)n, cudaMemcpyHostToDevice, st));
     GBP_CUDA(cudaEventRecord(c->ev[0], st));
     long long launches = 0;
-    GBP_CUDA(csr_cg_run(w, n, residual, max_iterations, c->grid_blocks, st, &launches));
+    const CgDebug debug = c->csr_debug;
+    c->csr_debug = {};  // one solve only
+    GBP_CUDA(csr_cg_run(w, n, residual, max_iterations, c->grid_blocks, debug, st, &launches));
+    if (w.host_sc->status == 4) return fail(GBP_ERR_CUDA, "gbp_csr_cg: a wait between the blocks of the solve ran out");
     GBP_CUDA(cudaEventRecord(c->ev[1], st));
     GBP_CUDA(cudaMemcpyAsync(x, w.x, sizeof(double) * (size_t)n, cudaMemcpyDeviceToHost, st));
     GBP_CUDA(cudaStreamSynchronize(st));
@@ -921,6 +925,15 @@ int gbp_debug_fail_wait(gbp_scene *s, int what, int block, int polls) {
         return fail(GBP_ERR_INVALID_ARGUMENT, "gbp_debug_fail_wait: what must be GBP_WAIT_GRID_BARRIER or "
                                               "GBP_WAIT_TILE, block >= 0 and polls in [1, 2^24]");
     s->solver->set_wait_test(what, block, polls);
+    return GBP_OK;
+}
+
+int gbp_debug_cg(gbp_ctx *c, gbp_scene *s, int launched, int steps, int block, int polls) {
+    if (!c || (s && (!s->solver || s->ctx != c)) || steps < 0 || block < 0 || polls < 0 || polls > (1 << 22))
+        return fail(GBP_ERR_INVALID_ARGUMENT, "gbp_debug_cg: NULL context, a scene of another, or a value out of range");
+    const CgDebug d{launched, steps, block, polls};
+    if (s) s->solver->set_cg_debug(d);
+    else c->csr_debug = d;
     return GBP_OK;
 }
 

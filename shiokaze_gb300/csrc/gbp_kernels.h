@@ -92,9 +92,16 @@ cudaError_t launch_cg_iteration(const Grid &g, Operator<double> A, double *x, do
 // with sc->done or after a few thousand iterations (status 4: a wait between
 // blocks ran out).
 constexpr int CG_PERSISTENT_STEPS = 4096;  // iterations in one launch
-bool cg_persistent_fits(const Grid &g, int grid_blocks);
+// What gbp_debug_cg asks of a solve; all zero in every ordinary one.
+struct CgDebug {
+    int launched = 0;  // nonzero: the launched iterations
+    int steps = 0;     // iterations of a launch of the one-launch form
+    int block = 0;     // with polls > 0: this block leaves out its arrivals
+    int polls = 0;     // ... and every wait polls at most this often
+};
+bool cg_persistent_fits(const Grid &g, int grid_blocks, const CgDebug &debug);
 cudaError_t launch_cg_persistent(const Grid &g, Operator<double> A, double *x, double *r, double *s, Scalars *sc,
-                                 Partials *pt, int grid_blocks, cudaStream_t stream);
+                                 Partials *pt, int grid_blocks, const CgDebug &debug, cudaStream_t stream);
 // The three launches of an iteration, one at a time (benchmarking).
 cudaError_t launch_cg_spmv(const Grid &g, Operator<double> A, const double *s, double *z, Scalars *sc, Partials *pt,
                            int grid_blocks, cudaStream_t stream);

@@ -294,10 +294,12 @@ int Solver::solve_cg(const Grid &grid, const gbp_params &p, int grid_blocks, cud
     SOLVER_CUDA(launch_cg_init(g, A, st_.b, warm ? st_.prev : nullptr, st_.x, st_.r, st_.s, st_.sc, st_.pt,
                                p.residual, p.max_iterations, grid_blocks, stream));
     *launches += 1;
-    if (cg_persistent_fits(g, grid_blocks)) {
+    const CgDebug debug = cg_debug_;
+    cg_debug_ = {};  // one solve only
+    if (cg_persistent_fits(g, grid_blocks, debug)) {
         cudaError_t e = cudaSuccess;
-        for (int left = p.max_iterations; e == cudaSuccess; left -= CG_PERSISTENT_STEPS) {
-            e = launch_cg_persistent(g, A, st_.x, st_.r, st_.s, st_.sc, st_.pt, grid_blocks, stream);
+        for (int left = p.max_iterations; e == cudaSuccess; left -= debug.steps > 0 ? debug.steps : CG_PERSISTENT_STEPS) {
+            e = launch_cg_persistent(g, A, st_.x, st_.r, st_.s, st_.sc, st_.pt, grid_blocks, debug, stream);
             if (e != cudaSuccess) break;
             *launches += 1;
             SOLVER_CUDA(cudaMemcpyAsync(st_.host_sc, st_.sc, sizeof(Scalars), cudaMemcpyDeviceToHost, stream));

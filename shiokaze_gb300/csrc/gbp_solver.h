@@ -77,6 +77,8 @@ public:
     bool staged() const { return runner_key_ >= 0 && runner_.scene_staged(0); }
     // test hook of gbp_debug_fail_wait: the next MGPCG solve's waits run out
     void set_wait_test(int what, int block, int polls) { runner_.set_wait_test(what, block, polls); }
+    // test hook of gbp_debug_cg, for the next CG solve
+    void set_cg_debug(const CgDebug &d) { cg_debug_ = d; }
 
 private:
     int fail(int code, const std::string &m) {
@@ -112,6 +114,7 @@ private:
     // batch of one for the scene's own MGPCG solves
     BatchRunner runner_;
     long long runner_key_ = -1;
+    CgDebug cg_debug_;
 };
 
 }  // namespace gbp
