@@ -75,9 +75,12 @@ __device__ __forceinline__ double sum_range(const double *part, int begin, int c
     return block_sum(v, sh);
 }
 
+// The largest of partial maxima of magnitudes, by their bit patterns: a NaN
+// outranks every number.
 __device__ __forceinline__ double max_range(const double *part, int begin, int count, double *sh) {
     unsigned long long v = 0;
-    for (int t = threadIdx.x; t < count; t += blockDim.x) v = max(v, abs_bits(__ldcg(part + begin + t)));
+    for (int t = threadIdx.x; t < count; t += blockDim.x)
+        v = max(v, (unsigned long long)__double_as_longlong(__ldcg(part + begin + t)));
     return __longlong_as_double((long long)block_max_bits(v));
 }
 
@@ -485,7 +488,7 @@ template <class T> struct MaxSumAcc {
         s.add(xt, xt);
     }
     __device__ void store(double *sh, double *part, int idx, int n) {
-        const double bm = block_max(__longlong_as_double((long long)m), sh);
+        const double bm = __longlong_as_double((long long)block_max_bits(m));
         const double bs = s.block(sh);
         if (threadIdx.x == 0) {
             part[idx] = bm;
