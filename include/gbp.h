@@ -253,9 +253,11 @@ int gbp_bricks_expand(gbp_ctx *ctx, int nx, int ny, int nz, const gbp_bricks *in
  * once per iteration for the whole batch, over a work list of tiles of all
  * scenes, and the iterations are replayed from one CUDA graph; each scene
  * stops on its own stopping rule, and its reductions are its own (per
- * scene, in a fixed order for a given batch): its result matches its
- * single-scene solve up to the grouping of its dot-product partials. Replaces a loop of macpressuresolver3::project calls over
- * independent scenes. Scenes belong to `ctx`; the batch refers to them (it
+ * scene, in an order of the scene's own): its result has the same bits whatever
+ * the batch's other scenes, and matches its single-scene solve up to the grouping
+ * of its dot-product partials. (TMA-staged scenes, gbp_params.tma_staging: up to
+ * that grouping in either case.) Replaces a loop of
+ * macpressuresolver3::project calls over independent scenes. Scenes belong to `ctx`; the batch refers to them (it
  * does not own them) and keeps their per-scene state (warm start, volume
  * correction). params->solver must be GBP_SOLVER_MGPCG. */
 typedef struct gbp_batch gbp_batch;

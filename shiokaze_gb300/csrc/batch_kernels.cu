@@ -367,19 +367,81 @@ __device__ __forceinline__ int next_item(int w, int gs) {
     return (w & ((1 << gs) - 1)) ? w : w + (((int)gridDim.x - 1) << gs);
 }
 
-// Reduction over a work list with one partial per (block, scene): a block
-// walks its items (sorted by scene), accumulates a scene's cells in
-// `acc`, and flushes when the scene changes. The flush of block b for a
-// scene whose items lie in the groups [g0, g1] of the list (item_group) goes
-// to slot (b - g0) mod gridDim.x of the scene's range;
-// min(g1 - g0 + 1, gridDim.x) blocks flush per scene (never more than it has
-// items), and the one taking the scene's last ticket combines the slots in
-// slot order (deterministic for a given batch and grid).
-template <class T, class Acc, bool CLASSES = true, class Body, class Finish>
-__device__ __forceinline__ void reduce_items(const BSeg *__restrict__ segs, int nseg, int n, double *part,
-                                             const BLevel<T> *levels, const BScene<T> *scenes, int gate,
-                                             ItemCtx<T> &ctx, Body body, Finish finish) {
-    __shared__ double sh[BLOCK_THREADS / 32];
+// Reductions over a work list: a block walks its items (sorted by scene) and takes
+// a ticket for each scene, after its last item there; the one that takes the
+// scene's last ticket combines the partials. A scene whose items lie in the
+// groups [g0, g1] of the list (item_group) meets min(g1 - g0 + 1, gridDim.x)
+// blocks.
+
+// Sums of a list of several scenes have one partial an item, combined in item
+// order: they depend on the scene alone, not on its company, its place in the
+// list or the grid. A block holds the threads' values of up to HELD items in
+// shared memory and adds them with a warp an item. (One partial per block and
+// scene took its items from the list's groups, and so depended on all three; a
+// batch of 64 liquids took 49.4 ms with it, 51.0 here, and 53.8 with one partial
+// per block over items dealt one by one.) The list of a single scene has one
+// partial per block, its items w, w + grid, ...: the same bits where no block has
+// two (256^3 mixed with one an item 10.36 instead of 9.88 ms).
+// Acc may keep a maximum beside the sum (MAXS), as in max_items; the sums are at
+// part + n then. finish(item, visits, sums): visits blocks met the scene, which
+// has `sums` partial sums.
+constexpr int HELD = 4;
+template <class T, class Acc, class Body, class Finish>
+__device__ __forceinline__ void sum_items(const BSeg *__restrict__ segs, int nseg, int n, double *part,
+                                          const BLevel<T> *levels, const BScene<T> *scenes, int gate,
+                                          ItemCtx<T> &ctx, Body body, Finish finish) {
+    __shared__ double vals[HELD * TREE_PAD];
+    const int gs = item_group(n, nseg);
+    const int stride = gs ? 1 : (int)gridDim.x;  // between the items held
+    int cur = -1, held = 0, newest = 0, sgc = 0;
+    BItem first{};
+    Acc acc;
+    acc.reset();
+    T cls_next = class_at<T, false>(levels, segs, nseg, n, first_item(gs), 0);
+    for (int w = first_item(gs);; w = next_item(w, gs)) {
+        // one level per scene in a list: a new level is a new scene
+        const BItem it = w < n ? item_at(segs, nseg, w, sgc) : BItem{-1, 0, 0, 0, 0, 0};
+        const bool leaves = it.ref != cur;
+        if (held && (leaves || held == HELD || (gs && (w & ((1 << gs) - 1)) == 0))) {
+            __syncthreads();
+            const int j = threadIdx.x >> 5;
+            if (j < held) {
+                const double p = tree256(vals + j * TREE_PAD);
+                if ((threadIdx.x & 31) == 0) part[(Acc::MAXS ? n : 0) + newest - (held - 1 - j) * stride] = p;
+            }
+            __syncthreads();
+            held = 0;
+        }
+        if (leaves) {
+            if (cur >= 0 && !ctx.skip) {
+                const int B = gridDim.x, g0 = first.begin >> gs, g1 = (first.begin + first.count - 1) >> gs;
+                if constexpr (Acc::MAXS) acc.store_max(part, first.begin + ((int)blockIdx.x - g0 % B + B) % B);
+                finish(first, min(g1 - g0 + 1, B), nseg > 1 ? first.count : min(first.count, B));
+            }
+            if (w >= n) return;
+            refresh(ctx, cur, it, levels, scenes, gate);
+            first = it;
+            acc.reset();
+        }
+        const T cls = cls_next;
+        cls_next = class_next<T, false>(levels, segs, nseg, n, next_item(w, gs), sgc, it.ref, ctx.L.tcp);
+        if (ctx.skip) continue;
+        body(it, acc, cls);
+        if (nseg > 1 || next_item(w, gs) >= n) {
+            vals[held * TREE_PAD + tree_at(threadIdx.x)] = acc.sum();
+            acc.reset_sum();
+            ++held;
+            newest = nseg > 1 ? w : (int)blockIdx.x;
+        }
+    }
+}
+
+// A maximum is the same in any order: one partial per (block, scene), at slot
+// (b - g0) mod gridDim.x of the scene's range for block b.
+template <class T, class Acc, class Body, class Finish>
+__device__ __forceinline__ void max_items(const BSeg *__restrict__ segs, int nseg, int n, double *part,
+                                          const BLevel<T> *levels, const BScene<T> *scenes, int gate,
+                                          ItemCtx<T> &ctx, Body body, Finish finish) {
     int cur = -1;
     BItem first{};
     Acc acc;
@@ -388,22 +450,21 @@ __device__ __forceinline__ void reduce_items(const BSeg *__restrict__ segs, int 
     auto flush = [&]() {
         const int B = gridDim.x, g0 = first.begin >> gs, g1 = (first.begin + first.count - 1) >> gs;
         const int slot = (int)((((long long)blockIdx.x - g0) % B + B) % B);
-        acc.store(sh, part, first.begin + slot, n);
+        acc.store_max(part, first.begin + slot);
         finish(first, min(g1 - g0 + 1, B));
     };
     int sgc = 0;
-    T cls_next = CLASSES ? class_at<T, false>(levels, segs, nseg, n, first_item(gs), 0) : T(TILE_MIXED);
+    T cls_next = class_at<T, false>(levels, segs, nseg, n, first_item(gs), 0);
     for (int w = first_item(gs); w < n; w = next_item(w, gs)) {
         const BItem it = item_at(segs, nseg, w, sgc);
         const T cls = cls_next;
         if (it.ref != cur) {
-            // one level per scene in a list: a new level is a new scene
             if (cur >= 0 && !ctx.skip) flush();
             refresh(ctx, cur, it, levels, scenes, gate);
             first = it;
             acc.reset();
         }
-        if (CLASSES) cls_next = class_next<T, false>(levels, segs, nseg, n, next_item(w, gs), sgc, it.ref, ctx.L.tcp);
+        cls_next = class_next<T, false>(levels, segs, nseg, n, next_item(w, gs), sgc, it.ref, ctx.L.tcp);
         if (!ctx.skip) body(it, acc, cls);
     }
     if (cur >= 0 && !ctx.skip) flush();
@@ -413,17 +474,20 @@ __device__ __forceinline__ void reduce_items(const BSeg *__restrict__ segs, int 
 // FP32 path: FloatFloat::add_product (gbp_floatfloat.cuh: the product split
 // exactly by an FMA, TwoSum, renormalised after every term; a thread's n
 // terms within gamma_n^2 sum |a_i b_i|); a partial is converted to FP64 once,
-// when its block flushes, and partials add across threads and blocks in FP64. The
+// when its item or block ends, and partials add across threads and blocks in FP64. The
 // FP32 path then issues no FP64 instruction per cell (the FP64 pipe of this
 // GPU runs at a small fraction of its FP32 rate). It assumes |a b| stays
 // inside the FP32 range, as the FP32 inner solve does for its vectors.
-// store() publishes the block's partial(s) at slot idx of the list's
-// partials (a second partial, if any, at n + idx).
+// sum() is the thread's partial; store() (the staged kernels) adds the block's and
+// publishes it at slot idx of the list's partials, store_max() its maximum.
 template <class T> struct DotAcc;
 template <> struct DotAcc<double> {
+    static constexpr bool MAXS = false;
     double v;
     __device__ void reset() { v = 0.0; }
     __device__ void add(double a, double b) { v = fma(a, b, v); }
+    __device__ double sum() const { return v; }
+    __device__ void reset_sum() { reset(); }
     __device__ double block(double *sh) { return block_sum(v, sh); }
     __device__ void store(double *sh, double *part, int idx, int) {
         const double b = block(sh);
@@ -431,9 +495,12 @@ template <> struct DotAcc<double> {
     }
 };
 template <> struct DotAcc<float> {
+    static constexpr bool MAXS = false;
     FloatFloat f;
     __device__ void reset() { f.reset(); }
     __device__ void add(float a, float b) { f.add_product(a, b); }
+    __device__ double sum() const { return f.value_fp64(); }
+    __device__ void reset_sum() { reset(); }
     __device__ double block(double *sh) { return block_sum(f.value_fp64(), sh); }
     __device__ void store(double *sh, double *part, int idx, int) {
         const double b = block(sh);
@@ -448,7 +515,7 @@ template <> struct MaxAcc<double> {
     unsigned long long v;
     __device__ void reset() { v = 0ull; }
     __device__ void add(double x) { v = max(v, abs_bits(x)); }
-    __device__ void store(double *, double *part, int idx, int) {
+    __device__ void store_max(double *part, int idx) {
         const unsigned long long b = block_max_bits(v);
         if (threadIdx.x == 0) part[idx] = __longlong_as_double((long long)b);
     }
@@ -457,7 +524,7 @@ template <> struct MaxAcc<float> {
     float v;
     __device__ void reset() { v = 0.0f; }
     __device__ void add(float x) { v = fmaxf(v, fabsf(x)); }
-    __device__ void store(double *, double *part, int idx, int) {
+    __device__ void store_max(double *part, int idx) {
         __shared__ unsigned maxs[BLOCK_THREADS / 32];
         unsigned b = __reduce_max_sync(0xffffffffu, __float_as_uint(v));
         __syncthreads();
@@ -476,6 +543,7 @@ template <> struct MaxAcc<float> {
 // product's accumulation (float-float for T = float), which only reports
 // the L2 norm.
 template <class T> struct MaxSumAcc {
+    static constexpr bool MAXS = true;
     unsigned long long m;
     DotAcc<T> s;
     __device__ void reset() {
@@ -487,13 +555,11 @@ template <class T> struct MaxSumAcc {
         m = b > m ? b : m;
         s.add(xt, xt);
     }
-    __device__ void store(double *sh, double *part, int idx, int n) {
-        const double bm = __longlong_as_double((long long)block_max_bits(m));
-        const double bs = s.block(sh);
-        if (threadIdx.x == 0) {
-            part[idx] = bm;
-            part[n + idx] = bs;
-        }
+    __device__ double sum() const { return s.sum(); }
+    __device__ void reset_sum() { s.reset(); }
+    __device__ void store_max(double *part, int idx) {
+        const unsigned long long b = block_max_bits(m);
+        if (threadIdx.x == 0) part[idx] = __longlong_as_double((long long)b);
     }
 };
 
@@ -1202,7 +1268,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS, OCC)
     if (batch_idle(live)) return;
     __shared__ double shf[BLOCK_THREADS / 32];
     __shared__ ItemCtx<T> ctx;
-    reduce_items<T, DotAcc<T>>(
+    sum_items<T, DotAcc<T>>(
         segs, nseg, n, part, levels, scenes, gate, ctx,
         [&](const BItem &it, DotAcc<T> &acc, T cls) {
             const BLevel<T> L = ctx.L;  // registers: stores through generic pointers would force reloads from shared memory
@@ -1236,10 +1302,10 @@ __global__ void __launch_bounds__(BLOCK_THREADS, OCC)
                     pair_tile(L.g, it, plane);
             });
         },
-        [&](const BItem &it, int flushes) {
+        [&](const BItem &it, int visits, int sums) {
             Scalars *sc = ctx.S.sc;
-            if (item_last(&sc->counter[SITE_DOT], flushes)) {
-                const double rho_new = sum_range(part, it.begin, flushes, shf);
+            if (item_last(&sc->counter[SITE_DOT], visits)) {
+                const double rho_new = sum_range(part, it.begin, sums, shf);
                 if (threadIdx.x == 0) {
                     if (sc->first) {
                         sc->beta = 0.0;
@@ -1641,7 +1707,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS, OCC)
     if (batch_idle(live)) return;
     __shared__ double shf[BLOCK_THREADS / 32];
     __shared__ ItemCtx<T> ctx;
-    reduce_items<T, DotAcc<T>>(
+    sum_items<T, DotAcc<T>>(
         segs, nseg, n, part, levels, scenes, gate, ctx,
         [&](const BItem &it, DotAcc<T> &acc, T cls) {
             const BLevel<T> L = ctx.L;  // registers: stores through generic pointers would force reloads from shared memory
@@ -1671,10 +1737,10 @@ __global__ void __launch_bounds__(BLOCK_THREADS, OCC)
                     pair_tile(L.g, it, plane);
             });
         },
-        [&](const BItem &it, int flushes) {
+        [&](const BItem &it, int visits, int sums) {
             Scalars *sc = ctx.S.sc;
-            if (item_last(&sc->counter[SITE_SPMV], flushes)) {
-                const double pq = sum_range(part, it.begin, flushes, shf);
+            if (item_last(&sc->counter[SITE_SPMV], visits)) {
+                const double pq = sum_range(part, it.begin, sums, shf);
                 if (threadIdx.x == 0) {
                     sc->pap = pq;
                     sc->alpha = sc->rho / pq;
@@ -1702,7 +1768,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS, OCC)
     if (batch_idle(live)) return;
     __shared__ double shf[BLOCK_THREADS / 32];
     __shared__ ItemCtx<T> ctx;
-    reduce_items<T, DotAcc<T>>(
+    sum_items<T, DotAcc<T>>(
         segs, nseg, n, part, levels, scenes, gate, ctx,
         [&](const BItem &it, DotAcc<T> &acc, T cls) {
             const BLevel<T> L = ctx.L;  // registers: stores through generic pointers would force reloads from shared memory
@@ -1749,10 +1815,10 @@ __global__ void __launch_bounds__(BLOCK_THREADS, OCC)
                     pair_tile(L.g, it, plane);
             });
         },
-        [&](const BItem &it, int flushes) {
+        [&](const BItem &it, int visits, int sums) {
             Scalars *sc = ctx.S.sc;
-            if (item_last(&sc->counter[SITE_SPMV], flushes)) {
-                const double pq = sum_range(part, it.begin, flushes, shf);
+            if (item_last(&sc->counter[SITE_SPMV], visits)) {
+                const double pq = sum_range(part, it.begin, sums, shf);
                 if (threadIdx.x == 0) {
                     sc->pap = pq;
                     sc->alpha = sc->rho / pq;
@@ -1773,7 +1839,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS, OCC)
     if (__syncthreads_or(threadIdx.x == 0 && batch_idle(cnt))) return;
     __shared__ double shf[BLOCK_THREADS / 32];
     __shared__ ItemCtx<T> ctx;
-    reduce_items<T, MaxAcc<T>>(
+    max_items<T, MaxAcc<T>>(
         segs, nseg, n, part, levels, scenes, gate, ctx,
         [&](const BItem &it, MaxAcc<T> &acc, T cls) {
             const BLevel<T> L = ctx.L;  // registers: stores through generic pointers would force reloads from shared memory
@@ -1838,10 +1904,10 @@ __global__ void __launch_bounds__(BLOCK_THREADS, OCC)
                     pair_tile(L.g, it, plane);
             });
         },
-        [&](const BItem &it, int flushes) {
+        [&](const BItem &it, int visits) {
             Scalars *sc = ctx.S.sc;
-            if (item_last(&sc->counter[SITE_UPDATE], flushes)) {
-                const double res = max_range(part, it.begin, flushes, shf);
+            if (item_last(&sc->counter[SITE_UPDATE], visits)) {
+                const double res = max_range(part, it.begin, visits, shf);
                 if (threadIdx.x == 0) {
                     sc->first_update = 0;
                     sc->iter += 1;
@@ -1980,7 +2046,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 4) refine_residual_kernel(
     if (!initial && !__syncthreads_or(threadIdx.x == 0 && *(const volatile int *)&cnt->refine > 0)) return;
     __shared__ double shf[BLOCK_THREADS / 32];
     __shared__ ItemCtx<T> ctx;
-    reduce_items<T, MaxSumAcc<T>>(
+    sum_items<T, MaxSumAcc<T>>(
         segs, nseg, n, part, levels, scenes, initial ? -1 : 2, ctx,
         [&](const BItem &it, MaxSumAcc<T> &acc, T cls) {
             const BLevel<T> L = ctx.L;  // registers: stores through generic pointers would force reloads from shared memory
@@ -2080,11 +2146,11 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 4) refine_residual_kernel(
                 });
             });
         },
-        [&](const BItem &it, int flushes) {
+        [&](const BItem &it, int visits, int sums) {
             Scalars *sc = ctx.S.sc;
-            if (item_last(&sc->counter[SITE_REFINE], flushes)) {
-                const double res = max_range(part, it.begin, flushes, shf);
-                const double ss = sum_range(part + n, it.begin, flushes, shf);
+            if (item_last(&sc->counter[SITE_REFINE], visits)) {
+                const double res = max_range(part, it.begin, visits, shf);
+                const double ss = sum_range(part + n, it.begin, sums, shf);
                 if (threadIdx.x == 0) {
                     sc->aux[0] = res;
                     sc->aux[1] = sqrt(ss);
@@ -2258,7 +2324,7 @@ __device__ __forceinline__ float staged_nsum(int h, const Grid &g, int i, int j,
 // when the item two back has been consumed, every thread waits on the
 // stage's mbarrier (bounded), computes from shared memory, and writes its
 // results to global memory. Reductions (red_dot, spmv) flush per scene as
-// reduce_items does. A wait that runs out records cnt->bar_err = 2 and the
+// sum_items does for a single scene. A wait that runs out records cnt->bar_err = 2 and the
 // block leaves after letting its other copy land (bounded); the host then
 // abandons the solve.
 template <int KIND>

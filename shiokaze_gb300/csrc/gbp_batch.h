@@ -5,12 +5,12 @@
 // therefore serves all scenes of a batch (of uneven sizes and depths) at
 // once, and a CUDA graph of a few iterations serves the whole batch.
 //
-// Reductions are per scene and deterministic: each item writes its tile's
-// partial, takes a ticket from its scene's counter, and the item that takes
-// the scene's last ticket sums that scene's partials in item order. A
-// scene's result therefore does not depend on which other scenes share the
-// batch (the serving test checks this), and a single-scene solve is a batch
-// of one.
+// Reductions are per scene and deterministic: every item has a partial sum
+// (the blocks of a single scene's list one each over their items), each block
+// takes a ticket for a scene it met, and the one with the scene's last ticket
+// adds the partials in item order. A scene's result therefore does not depend on
+// which other scenes share the batch (tests/test_gpu_batch_company.py); a
+// single-scene solve is a batch of one.
 #pragma once
 
 #include <cuda.h>
