@@ -22,6 +22,7 @@
 // and write) = 72 B.
 #include <type_traits>
 
+#include "gbp_barrier.cuh"
 #include "gbp_batch.h"
 #include "gbp_convert.cuh"
 #include "gbp_floatfloat.cuh"
@@ -994,13 +995,13 @@ __global__ void __launch_bounds__(BLOCK_THREADS, OCC)
 
 // ---- coarse levels in two cooperative launches -------------------------------------
 
-// Grid-wide barrier of a cooperative launch (every block resident): each
-// block adds 1 to cnt->bar_count, never reset within a solve, and waits until
-// the count reaches the next multiple of the grid (one atomic and polls of the
+// Grid-wide barrier of a cooperative launch (every block resident): the blocks
+// add to cnt->bar_count, never reset within a solve, and wait until the count
+// reaches the barrier's end (gbp_barrier.cuh; one atomic and polls of the
 // same word; a reset and a separate generation word took two more trips to L2,
 // and a sleep between polls another 0.1 us: the two cooperative kernels went
-// from 50 to 42 us an iteration at 128^3, 155 to 123 us at 256^3). The wait is bounded (about a
-// second); a block whose wait runs out records cnt->bar_err and leaves the
+// from 50 to 42 us an iteration at 128^3, 155 to 123 us at 256^3). The wait is bounded (about two
+// seconds); a block whose wait runs out records cnt->bar_err and leaves the
 // kernel, the others run out the same way, and the host reports the error.
 __device__ __forceinline__ bool grid_barrier(BatchCounters *cnt) {
     __syncthreads();
@@ -1012,11 +1013,13 @@ __device__ __forceinline__ bool grid_barrier(BatchCounters *cnt) {
             good = 0;
         } else {
             unsigned seen;
-            asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(seen) : "l"(&cnt->bar_count) : "memory");
-            const unsigned target = (seen / gridDim.x + 1) * gridDim.x;
+            const unsigned step = barrier_step(blockIdx.x, gridDim.x);
+            asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], %2;"
+                         : "=r"(seen) : "l"(&cnt->bar_count), "r"(step) : "memory");
+            const unsigned end = barrier_end(seen, gridDim.x);
             const int limit = cnt->test_polls > 0 ? cnt->test_polls : (1 << 22);
-            ++seen;
-            for (int it = 0; seen < target; ++it) {
+            seen += step;
+            for (int it = 0; !barrier_reached(seen, end); ++it) {
                 if (it > limit) {
                     good = 0;
                     atomicExch(&cnt->bar_err, 1);

@@ -419,7 +419,7 @@ template <class T> int BatchRunner::tune_occupancy(cudaStream_t st, const std::s
                 return e;
             };
             float t[3] = {0.f, 0.f, 0.f};
-            // the barriers count in multiples of the grid
+            // the count's multiples are those of the grid (gbp_barrier.cuh)
             err = cudaMemsetAsync(&d_counters_->bar_count, 0, sizeof(unsigned), st);
             if (err == cudaSuccess) err = run();
             for (int r = 0; r < 3 && err == cudaSuccess; ++r) {

@@ -146,7 +146,7 @@ inline long long cell_tiles(const Grid &g) { return g.ntiles; }
 struct BatchCounters {
     int remaining;        // scenes not done
     int refine;           // scenes whose inner solve ended, awaiting refinement
-    unsigned bar_count;   // grid barriers of the coarse-level kernels: arrivals, a multiple of the grid between launches
+    unsigned bar_count;   // grid barriers of the coarse-level kernels: arrivals (gbp_barrier.cuh)
     int bar_err;          // a barrier wait ran out (the solve is abandoned)
     // test hook (gbp_debug_fail_wait), 0 in every ordinary solve: block
     // test_block of the kernels named by test_what (1: the cooperative
