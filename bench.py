@@ -445,6 +445,8 @@ def run_gbp(args):
                 "algorithmic_bytes_per_launch": nbytes, "ms_per_launch": round(ms, 5),
                 "kernels": {n: {"ms": round(t[0], 5), "GBps": round(t[1] / (t[0] * 1e-3) / 1e9, 1)}
                             for n, t in timed.items()}}
+    if args.solver == "cg" and main["launches"] < args.steps * stats["iterations"]:
+        roofline["note"] = "kernels of the launched iterations; these solves ran in one launch each, without them"
 
     ms_step = total_ms / args.steps
     per_step = main["per_step"]

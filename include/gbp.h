@@ -310,7 +310,9 @@ int gbp_debug_cg(gbp_ctx *ctx, gbp_scene *scene, int launched, int steps, int bl
  * the mean milliseconds per launch and the algorithmic DRAM bytes one launch
  * moves (compulsory traffic over the dense grid). The scene's solver vectors
  * are overwritten; the next gbp_project recomputes them. No counterpart in
- * the reference (its timers are per phase, src/core/scoped_timer.cpp). */
+ * the reference (its timers are per phase, src/core/scoped_timer.cpp).
+ * The CG kernels are those of a solve's launched iterations; a system that fits
+ * the SMs' shared memory is solved in one launch without them. */
 #define GBP_KERNEL_CG_SPMV 0
 #define GBP_KERNEL_CG_UPDATE 1
 #define GBP_KERNEL_CG_DIRECTION 2

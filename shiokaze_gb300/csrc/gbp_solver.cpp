@@ -284,11 +284,15 @@ int Solver::complete(const Grid &g, const gbp_params &p, int grid_blocks, cudaSt
     return GBP_OK;
 }
 
+namespace {
+// CG's tiles stay one plane deep below 2^21 cells: they give its sums their
+// order, which decides (through CG's growth of rounding differences) where a
+// solve stops
+Grid cg_grid(const Grid &g) { return make_grid(g.dim, g.nx, g.ny, g.nz, DEEP_MIN_CG); }
+}  // namespace
+
 int Solver::solve_cg(const Grid &grid, const gbp_params &p, int grid_blocks, cudaStream_t stream, long long *launches) {
-    // CG's tiles stay one plane deep below 2^21 cells: they give its sums their
-    // order, which decides (through CG's growth of rounding differences) where
-    // a solve stops
-    const Grid g = make_grid(grid.dim, grid.nx, grid.ny, grid.nz, DEEP_MIN_CG);
+    const Grid g = cg_grid(grid);
     const bool warm = p.warm_start && st_.have_prev;
     Operator<double> A{st_.diag, st_.cx, st_.cy, g.dim == 3 ? st_.cz : st_.cy};
     SOLVER_CUDA(launch_cg_init(g, A, st_.b, warm ? st_.prev : nullptr, st_.x, st_.r, st_.s, st_.sc, st_.pt,
@@ -543,6 +547,7 @@ int Solver::bench_kernel(const Grid &g, int which, int reps, int grid_blocks, cu
     h.fluid_exists = 1;
     SOLVER_CUDA(cudaMemcpyAsync(st_.sc, &h, sizeof(h), cudaMemcpyHostToDevice, stream));
     Operator<double> A{st_.diag, st_.cx, st_.cy, g.dim == 3 ? st_.cz : st_.cy};
+    const Grid cg = cg_grid(g);
     const double cells = (double)g.ncell;
     const bool mixed = last_precision_ == GBP_PRECISION_MIXED;
     const double s = mixed ? 4.0 : 8.0;
@@ -551,15 +556,15 @@ int Solver::bench_kernel(const Grid &g, int which, int reps, int grid_blocks, cu
     switch (which) {
     case GBP_KERNEL_CG_SPMV:
         per_cell = 48.0;
-        launch = [&]() { return launch_cg_spmv(g, A, st_.s, st_.z, st_.sc, st_.pt, grid_blocks, stream); };
+        launch = [&]() { return launch_cg_spmv(cg, A, st_.s, st_.z, st_.sc, st_.pt, grid_blocks, stream); };
         break;
     case GBP_KERNEL_CG_UPDATE:
         per_cell = 48.0;
-        launch = [&]() { return launch_cg_update(g, st_.x, st_.r, st_.s, st_.z, st_.sc, st_.pt, grid_blocks, stream); };
+        launch = [&]() { return launch_cg_update(cg, st_.x, st_.r, st_.s, st_.z, st_.sc, st_.pt, grid_blocks, stream); };
         break;
     case GBP_KERNEL_CG_DIRECTION:
         per_cell = 24.0;
-        launch = [&]() { return launch_cg_direction(g, st_.r, st_.s, st_.sc, grid_blocks, stream); };
+        launch = [&]() { return launch_cg_direction(cg, st_.r, st_.s, st_.sc, grid_blocks, stream); };
         break;
     case GBP_KERNEL_MG_PRESMOOTH:
     case GBP_KERNEL_MG_RESTRICT:
