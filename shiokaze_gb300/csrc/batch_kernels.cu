@@ -70,15 +70,15 @@ __device__ __forceinline__ bool item_last(unsigned int *counter, int count) {
     return is_last;
 }
 
-__device__ __forceinline__ double sum_range(const double *part, int begin, int count, double *sh) {
+__device__ __forceinline__ double sum_range(const double *part, int begin, int count) {
     double v = 0.0;
     for (int t = threadIdx.x; t < count; t += blockDim.x) v += __ldcg(part + begin + t);
-    return block_sum(v, sh);
+    return block_sum(v);
 }
 
 // The largest of partial maxima of magnitudes, by their bit patterns: a NaN
 // outranks every number.
-__device__ __forceinline__ double max_range(const double *part, int begin, int count, double *sh) {
+__device__ __forceinline__ double max_range(const double *part, int begin, int count) {
     unsigned long long v = 0;
     for (int t = threadIdx.x; t < count; t += blockDim.x)
         v = max(v, (unsigned long long)__double_as_longlong(__ldcg(part + begin + t)));
@@ -489,9 +489,9 @@ template <> struct DotAcc<double> {
     __device__ void add(double a, double b) { v = fma(a, b, v); }
     __device__ double sum() const { return v; }
     __device__ void reset_sum() { reset(); }
-    __device__ double block(double *sh) { return block_sum(v, sh); }
-    __device__ void store(double *sh, double *part, int idx, int) {
-        const double b = block(sh);
+    __device__ double block() { return block_sum(v); }
+    __device__ void store(double *part, int idx) {
+        const double b = block();
         if (threadIdx.x == 0) part[idx] = b;
     }
 };
@@ -502,9 +502,9 @@ template <> struct DotAcc<float> {
     __device__ void add(float a, float b) { f.add_product(a, b); }
     __device__ double sum() const { return f.value_fp64(); }
     __device__ void reset_sum() { reset(); }
-    __device__ double block(double *sh) { return block_sum(f.value_fp64(), sh); }
-    __device__ void store(double *sh, double *part, int idx, int) {
-        const double b = block(sh);
+    __device__ double block() { return block_sum(f.value_fp64()); }
+    __device__ void store(double *part, int idx) {
+        const double b = block();
         if (threadIdx.x == 0) part[idx] = b;
     }
 };
@@ -1269,7 +1269,6 @@ __global__ void __launch_bounds__(BLOCK_THREADS, OCC)
                    const BScene<T> *__restrict__ scenes, int gate, double *part, const int *__restrict__ scene_of,
                    const BatchCounters *live) {
     if (batch_idle(live)) return;
-    __shared__ double shf[BLOCK_THREADS / 32];
     __shared__ ItemCtx<T> ctx;
     sum_items<T, DotAcc<T>>(
         segs, nseg, n, part, levels, scenes, gate, ctx,
@@ -1308,7 +1307,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS, OCC)
         [&](const BItem &it, int visits, int sums) {
             Scalars *sc = ctx.S.sc;
             if (item_last(&sc->counter[SITE_DOT], visits)) {
-                const double rho_new = sum_range(part, it.begin, sums, shf);
+                const double rho_new = sum_range(part, it.begin, sums);
                 if (threadIdx.x == 0) {
                     if (sc->first) {
                         sc->beta = 0.0;
@@ -1708,7 +1707,6 @@ __global__ void __launch_bounds__(BLOCK_THREADS, OCC)
                 const BScene<T> *__restrict__ scenes, int gate, double *part, const int *__restrict__ scene_of,
                 const BatchCounters *live) {
     if (batch_idle(live)) return;
-    __shared__ double shf[BLOCK_THREADS / 32];
     __shared__ ItemCtx<T> ctx;
     sum_items<T, DotAcc<T>>(
         segs, nseg, n, part, levels, scenes, gate, ctx,
@@ -1743,7 +1741,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS, OCC)
         [&](const BItem &it, int visits, int sums) {
             Scalars *sc = ctx.S.sc;
             if (item_last(&sc->counter[SITE_SPMV], visits)) {
-                const double pq = sum_range(part, it.begin, sums, shf);
+                const double pq = sum_range(part, it.begin, sums);
                 if (threadIdx.x == 0) {
                     sc->pap = pq;
                     sc->alpha = sc->rho / pq;
@@ -1769,7 +1767,6 @@ __global__ void __launch_bounds__(BLOCK_THREADS, OCC)
     direction_spmv_kernel(const BLevel<T> *__restrict__ levels, const BSeg *__restrict__ segs, int nseg, int n,
                           const BScene<T> *__restrict__ scenes, int gate, double *part, const BatchCounters *live) {
     if (batch_idle(live)) return;
-    __shared__ double shf[BLOCK_THREADS / 32];
     __shared__ ItemCtx<T> ctx;
     sum_items<T, DotAcc<T>>(
         segs, nseg, n, part, levels, scenes, gate, ctx,
@@ -1821,7 +1818,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS, OCC)
         [&](const BItem &it, int visits, int sums) {
             Scalars *sc = ctx.S.sc;
             if (item_last(&sc->counter[SITE_SPMV], visits)) {
-                const double pq = sum_range(part, it.begin, sums, shf);
+                const double pq = sum_range(part, it.begin, sums);
                 if (threadIdx.x == 0) {
                     sc->pap = pq;
                     sc->alpha = sc->rho / pq;
@@ -1840,7 +1837,6 @@ __global__ void __launch_bounds__(BLOCK_THREADS, OCC)
                   const int *__restrict__ scene_of) {
     // as in refine_residual_kernel: this launch lowers the counter
     if (__syncthreads_or(threadIdx.x == 0 && batch_idle(cnt))) return;
-    __shared__ double shf[BLOCK_THREADS / 32];
     __shared__ ItemCtx<T> ctx;
     max_items<T, MaxAcc<T>>(
         segs, nseg, n, part, levels, scenes, gate, ctx,
@@ -1910,7 +1906,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS, OCC)
         [&](const BItem &it, int visits) {
             Scalars *sc = ctx.S.sc;
             if (item_last(&sc->counter[SITE_UPDATE], visits)) {
-                const double res = max_range(part, it.begin, visits, shf);
+                const double res = max_range(part, it.begin, visits);
                 if (threadIdx.x == 0) {
                     sc->first_update = 0;
                     sc->iter += 1;
@@ -2047,7 +2043,6 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 4) refine_residual_kernel(
     // one thread decides for the block: the launch itself lowers the counter,
     // and a block whose warps disagreed would copy half of a descriptor
     if (!initial && !__syncthreads_or(threadIdx.x == 0 && *(const volatile int *)&cnt->refine > 0)) return;
-    __shared__ double shf[BLOCK_THREADS / 32];
     __shared__ ItemCtx<T> ctx;
     sum_items<T, MaxSumAcc<T>>(
         segs, nseg, n, part, levels, scenes, initial ? -1 : 2, ctx,
@@ -2152,8 +2147,8 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 4) refine_residual_kernel(
         [&](const BItem &it, int visits, int sums) {
             Scalars *sc = ctx.S.sc;
             if (item_last(&sc->counter[SITE_REFINE], visits)) {
-                const double res = max_range(part, it.begin, visits, shf);
-                const double ss = sum_range(part + n, it.begin, sums, shf);
+                const double res = max_range(part, it.begin, visits);
+                const double ss = sum_range(part + n, it.begin, sums);
                 if (threadIdx.x == 0) {
                     sc->aux[0] = res;
                     sc->aux[1] = sqrt(ss);
@@ -2342,7 +2337,6 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1)
     __shared__ __align__(8) unsigned long long bar[2];
     __shared__ int valid[2];
     __shared__ ItemCtx<float> ctx;
-    __shared__ double shf[BLOCK_THREADS / 32];
     float *stage0 = reinterpret_cast<float *>(st_smem + ((128u - (smem_u32(st_smem) & 127u)) & 127u));
     const int tid = threadIdx.x, G = gridDim.x;
     if (tid == 0) {
@@ -2407,12 +2401,12 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1)
     acc.reset();
     auto flush = [&]() {
         const int slot = (int)((((long long)blockIdx.x - first.begin) % G + G) % G);
-        acc.store(shf, part, first.begin + slot, n);
+        acc.store(part, first.begin + slot);
         const int flushes = min(first.count, G);
         Scalars *sc = ctx.S.sc;
         if constexpr (KIND == STAGE_RED_DOT) {
             if (item_last(&sc->counter[SITE_DOT], flushes)) {
-                const double rho_new = sum_range(part, first.begin, flushes, shf);
+                const double rho_new = sum_range(part, first.begin, flushes);
                 if (threadIdx.x == 0) {
                     if (sc->first) {
                         sc->beta = 0.0;
@@ -2430,7 +2424,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1)
             }
         } else if constexpr (KIND == STAGE_SPMV) {
             if (item_last(&sc->counter[SITE_SPMV], flushes)) {
-                const double pq = sum_range(part, first.begin, flushes, shf);
+                const double pq = sum_range(part, first.begin, flushes);
                 if (threadIdx.x == 0) {
                     sc->pap = pq;
                     sc->alpha = sc->rho / pq;

@@ -59,7 +59,6 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 6) cg_init_kernel(Grid g, Opera
                                                                 const double *__restrict__ prev, double *x, double *r,
                                                                 double *s, Scalars *sc, Partials *pt,
                                                                 double residual, int max_iter) {
-    __shared__ double sh[BLOCK_THREADS / 32];
     unsigned long long mx = 0;
     double r2 = 0.0;
     for_each_cell(g, [&](int i, int j, int k, long long c) {
@@ -72,14 +71,14 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 6) cg_init_kernel(Grid g, Opera
         r2 = fma(rv, rv, r2);
     });
     double bm = __longlong_as_double((long long)block_max_bits(mx));
-    double bs = block_sum(r2, sh);
+    double bs = block_sum(r2);
     if (threadIdx.x == 0) {
         pt->a[blockIdx.x] = bm;
         pt->b[blockIdx.x] = bs;
     }
     if (last_block(&sc->counter[0])) {
-        double res0 = reduce_partials_max(pt->a, gridDim.x, sh);
-        double rho = reduce_partials_sum(pt->b, gridDim.x, sh);
+        double res0 = reduce_partials_max(pt->a, gridDim.x);
+        double rho = reduce_partials_sum(pt->b, gridDim.x);
         if (threadIdx.x == 0) {
             double tolf = residual < 1e-30 ? 1e-30 : residual;  // pcg_solver.h:51
             sc->res0 = res0;
@@ -112,17 +111,16 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 6) cg_spmv_kernel(Grid g, Opera
                                                                 const double *__restrict__ s, double *z, Scalars *sc,
                                                                 Partials *pt) {
     if (stopped(sc)) return;
-    __shared__ double sh[BLOCK_THREADS / 32];
     double dot = 0.0;
     for_each_cell(g, [&](int i, int j, int k, long long c) {
         double zv = apply_A(g, A, s, i, j, k, c);
         z[c] = zv;
         dot = fma(__ldg(s + c), zv, dot);
     });
-    double bs = block_sum(dot, sh);
+    double bs = block_sum(dot);
     if (threadIdx.x == 0) pt->a[blockIdx.x] = bs;
     if (last_block(&sc->counter[1])) {
-        double pap = reduce_partials_sum(pt->a, gridDim.x, sh);
+        double pap = reduce_partials_sum(pt->a, gridDim.x);
         if (threadIdx.x == 0) {
             sc->pap = pap;
             sc->alpha = sc->rho / pap;
@@ -136,7 +134,6 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 6) cg_update_kernel(Grid g, dou
                                                                   const double *__restrict__ z, Scalars *sc,
                                                                   Partials *pt) {
     if (stopped(sc)) return;
-    __shared__ double sh[BLOCK_THREADS / 32];
     const double alpha = sc->alpha;
     unsigned long long mx = 0;
     double r2 = 0.0;
@@ -148,14 +145,14 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 6) cg_update_kernel(Grid g, dou
         r2 = fma(rv, rv, r2);
     });
     double bm = __longlong_as_double((long long)block_max_bits(mx));
-    double bs = block_sum(r2, sh);
+    double bs = block_sum(r2);
     if (threadIdx.x == 0) {
         pt->b[blockIdx.x] = bm;
         pt->c[blockIdx.x] = bs;
     }
     if (last_block(&sc->counter[2])) {
-        double res = reduce_partials_max(pt->b, gridDim.x, sh);
-        double rho_new = reduce_partials_sum(pt->c, gridDim.x, sh);
+        double res = reduce_partials_max(pt->b, gridDim.x);
+        double rho_new = reduce_partials_sum(pt->c, gridDim.x);
         if (threadIdx.x == 0) {
             sc->res = res;
             sc->r2 = rho_new;
@@ -191,7 +188,6 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 6) true_residual_kernel(Grid g,
                                                                       const double *__restrict__ x,
                                                                       const double *__restrict__ prev, Scalars *sc,
                                                                       Partials *pt) {
-    __shared__ double sh[BLOCK_THREADS / 32];
     unsigned long long mx = 0;
     double r2 = 0.0, b2 = 0.0;
     const long long sy = g.nx, sz = (long long)g.nx * g.ny;
@@ -226,17 +222,17 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 6) true_residual_kernel(Grid g,
         b2 = fma(b0, b0, b2);
     });
     double bm = __longlong_as_double((long long)block_max_bits(mx));
-    double bs = block_sum(r2, sh);
-    double bb = block_sum(b2, sh);
+    double bs = block_sum(r2);
+    double bb = block_sum(b2);
     if (threadIdx.x == 0) {
         pt->a[blockIdx.x] = bm;
         pt->b[blockIdx.x] = bs;
         pt->c[blockIdx.x] = bb;
     }
     if (last_block(&sc->counter[3])) {
-        double m = reduce_partials_max(pt->a, gridDim.x, sh);
-        double s2 = reduce_partials_sum(pt->b, gridDim.x, sh);
-        double sb = reduce_partials_sum(pt->c, gridDim.x, sh);
+        double m = reduce_partials_max(pt->a, gridDim.x);
+        double s2 = reduce_partials_sum(pt->b, gridDim.x);
+        double sb = reduce_partials_sum(pt->c, gridDim.x);
         if (threadIdx.x == 0) {
             sc->aux[0] = m;
             sc->aux[1] = sqrt(s2);

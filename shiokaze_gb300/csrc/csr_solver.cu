@@ -28,7 +28,6 @@ template <class F> __device__ __forceinline__ void for_each_row(long long n, F f
 __global__ void __launch_bounds__(BLOCK_THREADS) csr_init_kernel(long long n, const double *__restrict__ b, double *x,
                                                                  double *r, double *s, Scalars *sc, Partials *pt,
                                                                  double residual, int max_iter) {
-    __shared__ double sh[BLOCK_THREADS / 32];
     unsigned long long mx = 0;
     double r2 = 0.0;
     for_each_row(n, [&](long long row) {
@@ -40,14 +39,14 @@ __global__ void __launch_bounds__(BLOCK_THREADS) csr_init_kernel(long long n, co
         r2 = fma(rv, rv, r2);
     });
     const double bm = __longlong_as_double((long long)block_max_bits(mx));
-    const double bs = block_sum(r2, sh);
+    const double bs = block_sum(r2);
     if (threadIdx.x == 0) {
         pt->a[blockIdx.x] = bm;
         pt->b[blockIdx.x] = bs;
     }
     if (last_block(&sc->counter[0])) {
-        const double res0 = reduce_partials_max(pt->a, gridDim.x, sh);
-        const double rho = reduce_partials_sum(pt->b, gridDim.x, sh);
+        const double res0 = reduce_partials_max(pt->a, gridDim.x);
+        const double rho = reduce_partials_sum(pt->b, gridDim.x);
         if (threadIdx.x == 0) {
             const double tolf = residual < 1e-30 ? 1e-30 : residual;  // pcg_solver.h:240
             sc->res0 = res0;
@@ -84,7 +83,6 @@ __global__ void __launch_bounds__(BLOCK_THREADS) csr_spmv_kernel(long long n, co
                                                                  const double *__restrict__ s, double *z, Scalars *sc,
                                                                  Partials *pt) {
     if (stopped(sc)) return;
-    __shared__ double sh[BLOCK_THREADS / 32];
     double dot = 0.0;
     for_each_row(n, [&](long long row) {
         const long long e0 = __ldg(rowstart + row), e1 = __ldg(rowstart + row + 1);
@@ -93,10 +91,10 @@ __global__ void __launch_bounds__(BLOCK_THREADS) csr_spmv_kernel(long long n, co
         z[row] = acc;
         dot = fma(__ldg(s + row), acc, dot);
     });
-    const double bs = block_sum(dot, sh);
+    const double bs = block_sum(dot);
     if (threadIdx.x == 0) pt->a[blockIdx.x] = bs;
     if (last_block(&sc->counter[1])) {
-        const double pap = reduce_partials_sum(pt->a, gridDim.x, sh);
+        const double pap = reduce_partials_sum(pt->a, gridDim.x);
         if (threadIdx.x == 0) {
             sc->pap = pap;
             sc->alpha = sc->rho / pap;
@@ -112,7 +110,6 @@ __global__ void __launch_bounds__(BLOCK_THREADS) csr_update_kernel(long long n, 
                                                                    const double *__restrict__ z, Scalars *sc,
                                                                    Partials *pt) {
     if (stopped(sc)) return;
-    __shared__ double sh[BLOCK_THREADS / 32];
     const double alpha = sc->alpha;
     unsigned long long mx = 0;
     double r2 = 0.0;
@@ -124,14 +121,14 @@ __global__ void __launch_bounds__(BLOCK_THREADS) csr_update_kernel(long long n, 
         r2 = fma(rv, rv, r2);
     });
     const double bm = __longlong_as_double((long long)block_max_bits(mx));
-    const double bs = block_sum(r2, sh);
+    const double bs = block_sum(r2);
     if (threadIdx.x == 0) {
         pt->b[blockIdx.x] = bm;
         pt->c[blockIdx.x] = bs;
     }
     if (last_block(&sc->counter[2])) {
-        const double res = reduce_partials_max(pt->b, gridDim.x, sh);
-        const double rho_new = reduce_partials_sum(pt->c, gridDim.x, sh);
+        const double res = reduce_partials_max(pt->b, gridDim.x);
+        const double rho_new = reduce_partials_sum(pt->c, gridDim.x);
         if (threadIdx.x == 0) {
             sc->res = res;
             sc->r2 = rho_new;

@@ -207,7 +207,7 @@ __device__ __forceinline__ unsigned long long warp_max_bits(unsigned long long b
 }
 
 // Block-wide sum in a fixed order; result valid in thread 0.
-__device__ __forceinline__ double block_sum(double v, double *) {
+__device__ __forceinline__ double block_sum(double v) {
     __shared__ double vals[TREE_PAD];
     __syncthreads();
     vals[tree_at(threadIdx.x)] = v;
@@ -223,11 +223,6 @@ __device__ __forceinline__ unsigned long long block_max_bits(unsigned long long 
     if ((threadIdx.x & 31) == 0) maxs[threadIdx.x >> 5] = b;
     __syncthreads();
     return threadIdx.x < 32 ? warp_max_bits(threadIdx.x < BLOCK_THREADS / 32 ? maxs[threadIdx.x] : 0ull) : 0ull;
-}
-
-// Block-wide maximum of |v|, NaN ignored; result valid in warp 0.
-__device__ __forceinline__ double block_max(double v, double *) {
-    return __longlong_as_double((long long)block_max_bits(abs_bits(v)));
 }
 
 // Publishes this block's partial(s) and returns true in every thread of the
@@ -247,13 +242,13 @@ __device__ __forceinline__ bool last_block(unsigned int *counter) {
 
 // Sums partial[0..n) in a fixed order (strided per thread, then the block
 // tree); result valid in thread 0.
-__device__ __forceinline__ double reduce_partials_sum(const double *partial, int n, double *sh) {
+__device__ __forceinline__ double reduce_partials_sum(const double *partial, int n) {
     double v = 0.0;
     for (int t = threadIdx.x; t < n; t += blockDim.x) v += __ldcg(partial + t);
-    return block_sum(v, sh);
+    return block_sum(v);
 }
 
-__device__ __forceinline__ double reduce_partials_max(const double *partial, int n, double *sh) {
+__device__ __forceinline__ double reduce_partials_max(const double *partial, int n) {
     unsigned long long v = 0;
     for (int t = threadIdx.x; t < n; t += blockDim.x) v = max(v, abs_bits(__ldcg(partial + t)));
     return __longlong_as_double((long long)block_max_bits(v));
