@@ -132,6 +132,11 @@ struct CsrRows {
     }
 };
 
+// x != x without an FP64 instruction on the iteration's critical path
+__device__ __forceinline__ bool nan_bits(double x) {
+    return ((unsigned long long)__double_as_longlong(x) << 1) > 0xffe0000000000000ull;
+}
+
 // All blocks; false if a wait ran out. Writes before it are visible after it.
 // TEST: block a.fail_block leaves instead of arriving, waits poll a.polls times.
 template <bool CLUSTER, bool TEST>
@@ -318,7 +323,7 @@ __global__ void __launch_bounds__(CLUSTER ? 512 : 768, 1) cg_persistent_kernel(c
         if (tid == 0) {
             r2 = rho_new;
             // NaN first: |r|_inf and the marks pass over it (a NaN's sign says nothing)
-            sh_status = rho_new != rho_new || alpha != alpha ? 3 : (!more ? 1 : (iter >= max_iter ? 2 : 0));
+            sh_status = nan_bits(rho_new) || nan_bits(alpha) ? 3 : (!more ? 1 : (iter >= max_iter ? 2 : 0));
             sh_scalar = rho_new / rho;
             if (!sh_status) rho = rho_new;
         }
