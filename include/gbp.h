@@ -96,13 +96,17 @@ typedef struct gbp_params {
     int mg_coarsest;        /* coarsen while any edge exceeds this (default 7) */
     double inner_tolerance; /* MIXED: relative residual of each inner solve (default 1e-3) */
     int iterations_per_sync;/* CG iterations between host checks of convergence (default 16); a solve that fits the
-                               SMs' shared memory runs in one launch and checks every iteration on the device */
+                               SMs' shared memory runs in one launch of up to 4096 iterations, which checks
+                               every iteration on the device and holds all SMs (16 in a cluster for up to
+                               64 tiles): other streams' kernels may wait for it, up to 0.1 s at 800,000 cells */
     double surface_tension; /* the surface_tension argument of macproject3_interface::project
                                (macpressuresolver3.cpp:85-115); 0 (default) leaves the velocity as is */
     int tma_staging;        /* MGPCG MIXED: nonzero runs the fine level's four stencil passes with their
                                tiles staged in shared memory by TMA where the grid allows it (3D, at least
                                2^21 cells, nx % 8 == 0); 0 (default) uses the direct-load kernels, which
-                               compute every cell alike and measure faster over a whole solve on GB300 */
+                               measure faster over a whole solve on GB300. The two agree up to rounding: the
+                               staged form smooths after prolongation from b and the neighbours' values and
+                               forms A p from p, the other adds the correction's effect and A p's recurrence */
     int tile_classes;       /* MGPCG: nonzero (default) lets the multigrid and CG kernels use the tile classes of
                                each level: in the FP32 kernels a tile whose couplings all share one value reads
                                that value instead of the coupling arrays, and a tile with no unknown writes zeros
@@ -284,8 +288,8 @@ int gbp_debug_assemble(gbp_scene *scene, double dt, const float *solid, const fl
  * grid-wide barriers of the cooperative coarse-level kernels;
  * GBP_WAIT_TILE: the copies of its first tile in the TMA-staged fine-level
  * kernels (gbp_params.tma_staging) -- and every bounded wait polls at most
- * `polls` times (1..2^24; the defaults are 2^24 and 2^22 polls, about a
- * second). The waits of the other blocks (or of that block) then run out,
+ * `polls` times (1..2^24; the default is 2^22 polls, about two
+ * seconds). The waits of the other blocks (or of that block) then run out,
  * the kernels record it and return, and the solve returns GBP_ERR_CUDA with
  * a message naming the wait; the context stays usable and the next solve
  * runs normally. Nothing faults and nothing waits without a limit. */

@@ -2,9 +2,10 @@
 // items spanning every scene of a batch (see gbp_batch.h).
 //
 // Red (i+j+k even) / black Gauss-Seidel, Galerkin restriction by summing the
-// 8 children's residuals, post-smoothing black (reading the red neighbours
-// with their parent's correction added) then red, a shared-memory tail per
-// scene for the small levels, and CG with FP64-accumulated dot products.
+// 4 red children's residuals (the black ones' are zero after the pre-smoothing),
+// post-smoothing black (adding the coarse correction's effect alone) then red, a
+// tail of one block per scene for the small levels, and CG with
+// FP64-accumulated dot products.
 //
 // Every kernel walks pair tiles (64 x 8 x tz cells): a thread owns the two
 // x-adjacent cells (i, i+1) of a row, i even, one of each colour. On levels
@@ -1326,10 +1327,10 @@ __global__ void __launch_bounds__(BLOCK_THREADS, OCC)
         });
 }
 
-// ---- shared-memory tail, one block per scene -----------------------------------
+// ---- tail, one block per scene --------------------------------------------------
 
-// A tail level in shared memory; descriptors live in shared memory too (one
-// copy per block, read as broadcasts).
+// A tail level, in place in global memory; its descriptor lives in shared memory
+// (one copy per block, read as broadcasts).
 template <class T> struct SLevel {
     int nx, ny, nz, dim, n;
     int hx;             // pair slots per row, (nx + 1) / 2
@@ -2268,7 +2269,7 @@ __device__ __forceinline__ void mbar_init(unsigned long long *b) {
 __device__ __forceinline__ void mbar_expect(unsigned long long *b, unsigned bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(b)), "r"(bytes) : "memory");
 }
-// Bounded wait for the phase of the given parity (about a second at most
+// Bounded wait for the phase of the given parity (about two seconds at most
 // with the default limit of 2^22 polls).
 __device__ __forceinline__ bool mbar_wait(unsigned long long *b, unsigned parity, int limit) {
     for (int it = 0; it < limit; ++it) {

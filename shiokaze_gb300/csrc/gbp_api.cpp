@@ -57,7 +57,8 @@ void set_last_error(const std::string &msg) { g_last_error = msg; }
 // Those kernels are bound by the latency of a few cut faces' FP64 chains (87
 // us for the faces of a 90^3 liquid, 413 us for 256^3), which overlap between
 // scenes: a batch of 64 liquids took 69.4 ms on one stream, 61.6 ms on six, six
-// served scenes 26.9 and 24.5 ms.
+// served scenes 26.9 and 24.5 ms. (Later, with the iteration faster: three streams
+// 51.7 and 19.9 ms, six 50.9 and 19.8, twelve 50.8 and 20.1.)
 constexpr int kLanes = 6;
 
 struct gbp_ctx {

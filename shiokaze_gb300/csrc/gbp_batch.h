@@ -75,7 +75,7 @@ template <class T> struct BScene {
     double *x64, *r64;
     Scalars *sc;
     int levels;  // multigrid levels of the scene
-    int tail;    // first level of its shared-memory tail (== levels: none)
+    int tail;    // first level of its tail (== levels: none)
 };
 
 struct BItem {

@@ -31,7 +31,7 @@
 //   sweep (1 colour) read x, b, inv, cx, cy, cz (half the cells
 //                    written); counted as a full pass                 7 s
 //   restrict         read x, b, diag, cx, cy, cz; write b_c / 8      6 s + s/8
-//   post_black       read x, x_c / 8, b, inv, cx, cy, cz; write half x  7 s
+//   post_black       read x, x_c / 8, inv, cx, cy, cz; write half x  6 s + s/8
 //   direction, spmv  read z, p, q, half of r and of diag, cx, cy, cz;
 //                    write p, q                                       9 s
 //                    (staged levels, two passes: read z, p; write p, 3 s,
