@@ -173,7 +173,6 @@ cudaError_t csr_reserve(CsrWork &w, long long n, long long nnz) {
     cudaError_t e = cudaSuccess;
     if (!w.sc) {
         if ((e = cudaMalloc(&w.sc, sizeof(Scalars))) != cudaSuccess) return e;
-        if ((e = cudaMemset(w.sc, 0, sizeof(Scalars))) != cudaSuccess) return e;
         if ((e = cudaMalloc(&w.pt, sizeof(Partials))) != cudaSuccess) return e;
         if ((e = cudaMallocHost(&w.host_sc, sizeof(Scalars))) != cudaSuccess) return e;
     }
